@@ -317,7 +317,7 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct Layout {  // byte offsets inside the pool
   size_t cards[2], w[2], same[2], ops[2], steps[2], groups[2], nodes, board_cards, iso_perm[2], iso_off, iso_ent;  // static
-  size_t gidx[2], coff[2], thr[2], nvalid[2], heads[2];                                                       // setup
+  size_t ord[2], gt[2], thr[2], fold[2], nvalid[2];                                                           // setup
   size_t R, S, SG, ipcfv, chcfv, rootv[2];                                                              // state
   size_t bcfv, breach;  // boundary values and boundary reach (kept across state resets)
 };
@@ -470,11 +470,11 @@ struct Batch {
         L.steps[p] = take(so, g.prog[p].steps.size() * sizeof(Step));
         L.groups[p] = take(so, g.prog[p].groups.size() * 2 + 16);
         L.iso_perm[p] = take(so, g.iso_perm[p].size() * (size_t)g.hs[p] * 2 + 16);
-        L.gidx[p] = take(su, nb * 3 * g.hs[p] * 2);
-        L.coff[p] = take(su, nb * 56 * 2);
+        L.ord[p] = take(su, nb * g.hs[p] * 2);
+        L.gt[p] = take(su, nb * 16 * (size_t)gather_vecs(g.hs[p]));
         L.thr[p] = take(su, nb * g.hs[p] * kThrWords * 2);
+        L.fold[p] = take(su, nb * g.hs[p] * 8);
         L.nvalid[p] = take(su, nb * 4);
-        L.heads[p] = take(su, nb * 4 * (size_t)head_words(g.hs[p]));
       }
       L.nodes = take(so, g.arena.size() * sizeof(NodeDev));
       L.board_cards = take(so, nb * 5);
@@ -556,11 +556,11 @@ struct Batch {
         s.steps[p] = (const Step*)(dS + L.steps[p]);
         s.groups[p] = (const uint16_t*)(dS + L.groups[p]);
         s.iso_perm[p] = (const uint16_t*)(dS + L.iso_perm[p]);
-        s.gidx[p] = (uint16_t*)(dU + L.gidx[p]);
-        s.coff[p] = (uint16_t*)(dU + L.coff[p]);
+        s.ord[p] = (uint16_t*)(dU + L.ord[p]);
+        s.gt[p] = (uint16_t*)(dU + L.gt[p]);
         s.thr[p] = (uint16_t*)(dU + L.thr[p]);
+        s.fold[p] = (uint32_t*)(dU + L.fold[p]);
         s.nvalid[p] = (int32_t*)(dU + L.nvalid[p]);
-        s.heads[p] = (uint32_t*)(dU + L.heads[p]);
       }
       NodeDev* nd = (NodeDev*)(h_static + L.nodes);
       // reach scale of every node: the product of the rounded 1 / chance_factor
@@ -2112,7 +2112,7 @@ int ps_hand_strength(ps_game* G, int turn, int river, int p, uint16_t* strength,
   int V = 0;
   CU(cudaMemcpy(&V, s.nvalid[p] + b, 4, cudaMemcpyDeviceToHost));
   std::vector<uint16_t> ord(V), thr((size_t)g.hs[p] * kThrWords);
-  CU(cudaMemcpy(ord.data(), s.gidx[p] + (size_t)b * 3 * g.hs[p], 2 * (size_t)V, cudaMemcpyDeviceToHost));
+  CU(cudaMemcpy(ord.data(), s.ord[p] + (size_t)b * g.hs[p], 2 * (size_t)V, cudaMemcpyDeviceToHost));
   // the strength of each ordered hand: recover from the opponent's thresholds is
   // indirect, so evaluate it on the host with the shared evaluator
   std::vector<int32_t> table(kHandTableSize);
@@ -2145,7 +2145,7 @@ int ps_valid_indices(ps_game* G, int turn, int river, int p, uint16_t* out) {
   CU(cudaMemcpy(thr.data(), s.thr[p] + (size_t)b * g.hs[p] * kThrWords, 2 * thr.size(), cudaMemcpyDeviceToHost));
   int n = 0;
   for (int h = 0; h < g.H[p]; ++h)
-    if (thr[(size_t)h * kThrWords] != 0xFFFF || thr[(size_t)h * kThrWords + 1] != 0xFFFF) out[n++] = (uint16_t)h;
+    if (thr[(size_t)h * kThrWords] != 0) out[n++] = (uint16_t)h;  // a blocked hand's record is all zero
   return n;
 }
 

@@ -84,10 +84,10 @@ struct SpotDev {
   const uint16_t* groups[2];  // terminal-group leader offsets of every step
   const NodeDev* nodes;
   const uint8_t* board_cards; // [num_boards][5], 255 = none
-  uint16_t* gidx[2];   // opponent o: [num_boards][3 * hs[o]] gather order (ord, then by card)
-  uint16_t* coff[2];   // opponent o: [num_boards][56] card segment starts within the card part
+  uint16_t* ord[2];    // player: [num_boards][hs] hands in strength order
+  uint16_t* gt[2];     // opponent o: [num_boards][gather_vecs(hs[o])] 16-byte vectors of the gather table
   uint16_t* thr[2];    // player p: [num_boards][hs[p]] 16-byte lookup records vs the opponent
-  uint32_t* heads[2];  // opponent o: [num_boards][(3 * hs[o] + 31) / 32] segment-start bits of the gather list
+  uint32_t* fold[2];   // player p: [num_boards][hs[p]] 8-byte fold records vs the opponent
   int32_t* nvalid[2];  // player: [num_boards] valid hand count
   const float* bcfv;   // boundary cfvs [num_boundary][2][vstride] (pot-normalised)
   const uint16_t* iso_perm[2]; // player: [perm id][hs] index of the suit-swapped hand

@@ -39,7 +39,13 @@ constexpr int ERR_SCRATCH = 1;  // a spot needed more scratch than its CTA owns
 constexpr int ERR_SETUP = 2;    // setup tables exceeded their bounds
 constexpr int ERR_WAIT = 4;     // a grid barrier gave up waiting for the other CTAs
 
-constexpr uint32_t THR_INVALID = 0xFFFFFFFFu;
+// A blocked hand's lookup and fold records are all zero (a valid hand's first
+// position is at least kScanBase - 1, and its fold record carries FOLD_VALID):
+// every position then reads the zero below the scan list, so the lookup loops
+// need no branch around a blocked hand's loads.
+constexpr uint32_t FOLD_VALID = 0x80000000u, FOLD_SAME = 0x40000000u;
+// gather-table entry: byte offset of the reach value | GT_HEAD at a segment start
+constexpr uint32_t GT_HEAD = 0x8000u, GT_OFFSET = 0x7FFCu;
 
 // Optional per-phase cycle counters (build with -DPS_PHASE_TIMERS): lane 0 of
 // every warp adds the clock64 cycles it spent in each phase, so the totals
@@ -73,9 +79,9 @@ __device__ __forceinline__ float* shared_view(float* p) {
 }
 
 struct Tables {  // board tables of one board, in shared or global memory
-  const uint16_t* gidx[2];   // opponent-indexed gather lists
-  const uint32_t* heads[2];  // opponent-indexed segment-start bitmaps
-  const uint4* thr[2];       // player-indexed lookup records
+  const uint4* gt[2];     // opponent-indexed gather tables
+  const uint4* thr[2];    // player-indexed lookup records
+  const uint2* fold[2];   // player-indexed fold records
   int nvalid[2];
 };
 
@@ -405,36 +411,41 @@ __device__ __forceinline__ void board_tables(const Ctx& c, int b, Tables& t) {
   }
   const SpotDev& sp = *c.sp;
   for (int q = 0; q < 2; ++q) {
-    t.gidx[q] = sp.gidx[q] + (size_t)b * 3 * sp.hs[q];
-    t.heads[q] = sp.heads[q] + (size_t)b * head_words(sp.hs[q]);
+    t.gt[q] = reinterpret_cast<const uint4*>(sp.gt[q]) + (size_t)b * gather_vecs(sp.hs[q]);
     t.thr[q] = reinterpret_cast<const uint4*>(sp.thr[q]) + (size_t)b * sp.hs[q];
+    t.fold[q] = reinterpret_cast<const uint2*>(sp.fold[q]) + (size_t)b * sp.hs[q];
     t.nvalid[q] = sp.nvalid[q][b];
   }
 }
 
 // Evaluates a run of n terminals that read the same reach on the same board,
-// for traverser p, with the calling warp alone, in three phases whose memory
-// accesses are issued as independent batches:
-//  1. gather: every lane reads four gather indices at a time (16 entries per
-//     batch) and the opponent reach at those indices; a segment start is
-//     stored as -x (reach values are >= +0, so the sign bit flags a start even
-//     for a zero);
-//  2. scan: each lane scans a contiguous chunk of the 3V-entry list of odd
-//     length (the lanes' strided shared-memory accesses then fall in distinct
-//     banks), a segmented warp scan of the chunk totals gives each chunk its
-//     carry-in, and the chunk's entries before its first segment start add it;
-//  3. lookups: per terminal, every hand reads its 16-byte record and its
-//     win / lose / blocked sums at the recorded positions of the scan.
-// GEN = false is the copy the solve passes use (non-negative reach, the
-// traverser's own payoffs, no boundary gradients); GEN = true adds what the
-// average-strategy passes of root_cfvalues_with_reach and the adjoint need.
+// for traverser p, with the calling warp alone, in three phases:
+//  1. gather and scan: lane l sums entries [l C, (l + 1) C) of the 3V-entry
+//     list in order, restarting at segment starts, and stores each running sum
+//     at its list position (C is odd, so the lanes' strided stores fall in
+//     distinct banks).  The entries come from the board's gather table, which
+//     k_setup lays out by lane: one 16-byte load brings a lane eight entries
+//     (byte offset of the reach value, and whether it starts a segment), so a
+//     round's eight gathers are independent of each other and of the sums;
+//  2. a segmented warp scan of the chunk totals gives each chunk its carry-in,
+//     and the chunk's entries before its first segment start add it;
+//  3. lookups: per terminal, every hand reads its 16-byte record (8 bytes for a
+//     fold or a depth boundary) and its win / lose / blocked sums at the
+//     recorded positions of the scan, two hands per lane and round.
+// Bound by instruction issue and the latency of its dependent loads.  Against
+// the form with a separate gather into the buffer, a scan over it and one hand
+// per round (same sums, same bits): 4096 datagen river spots 613 -> 493 ms a
+// batch with its records, 1024 depth-limited turn spots 17.1 -> 12.2 ms per 10
+// iterations, their adjoint 8.0 -> 5.5 ms.
+// GEN = false is the copy the solve passes use (the traverser's own payoffs, no
+// boundary gradients); GEN = true adds what the average-strategy passes of
+// root_cfvalues_with_reach and the adjoint need.
 // SPLIT (solve passes of launches whose CTAs hold a lone spot): the run is
 // part c.part of c.parts warps; each gathers and scans the whole list in its
 // own buffer and evaluates the hands of its interleaved 32-hand blocks.
 // CTA (grid mode, every warp holding a buffer): the whole CTA evaluates the
-// run in warp 0's buffer.  All warps gather, warp 0 alone scans (the same
-// chunks, so the same sums), and warp w evaluates hand blocks w, w + W, ...;
-// every thread of the CTA calls it for the same runs.
+// run in warp 0's buffer.  Warp 0 gathers and scans, and warp w evaluates hand
+// blocks w, w + W, ...; every thread of the CTA calls it for the same runs.
 // Raked showdown value of one hand (evaluation.rs:429-537), out of line: the
 // solve loop of unraked trees never takes it, and the per-hand loop stays small.
 __device__ __noinline__ float raked_showdown_value(float cw, float cl, float ctie, float win, float Ple, float Q1le,
@@ -446,114 +457,123 @@ __device__ __noinline__ float raked_showdown_value(float cw, float cl, float cti
   return cw * win + ctie * (tie - win + rs) + cl * (tot - tie);
 }
 
+__device__ __forceinline__ float byte_at(const float* p, uint32_t off) {
+  return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + off);
+}
 
-#ifndef PS_GATHER_U
-#define PS_GATHER_U 2  // groups of four entries each lane gathers per round (2 measured best of 1-4)
-#endif
+// The scan buffer's prefix at a record's u16 position, and the win / lose sums
+// of a 16-byte record.  The caller has added the buffer's own position in the
+// dynamic shared memory (in floats, below 2^16 as is their sum) to both halves
+// of every word with one addition, so a prefix costs its unpacking and one
+// 32-bit shared load.
+__device__ __forceinline__ float pref_lo(const float* sm, uint32_t w) { return sm[w & 0xFFFFu]; }
+__device__ __forceinline__ float pref_hi(const float* sm, uint32_t w) { return sm[w >> 16]; }
+__device__ __forceinline__ float showdown_value(const float* sm, uint32_t bb, uint4 t, float Tsum, float cw,
+                                                float cl) {
+  const uint32_t x = t.x + bb, y = t.y + bb, z = t.z + bb, w = t.w + bb;
+  const float Plt = pref_lo(sm, x), Ple = pref_hi(sm, x);
+  const float Q1lt = pref_lo(sm, y), Q1le = pref_hi(sm, y);
+  const float M1 = pref_lo(sm, z), Q2lt = pref_hi(sm, z);
+  const float Q2le = pref_lo(sm, w), M2 = pref_hi(sm, w);
+  const float win = Plt - Q1lt - Q2lt;
+  const float lose = (Tsum - Ple) - (M1 - Q1le) - (M2 - Q2le);
+  const float v = __fadd_rn(__fmul_rn(cw, win), __fmul_rn(cl, lose));
+  return t.x ? v : 0.f;
+}
+// T + r_same - M_c1 - M_c2 of a fold record (0 for a blocked hand through the
+// caller's FOLD_VALID test); same(off): the weighted reach at a byte offset
+template <class Same>
+__device__ __forceinline__ float blocked_reach(const float* sm, uint32_t bb, uint2 f, float Tsum, Same same) {
+  const uint32_t x = f.x + bb;
+  const float M1 = pref_lo(sm, x), M2 = pref_hi(sm, x);
+  const float rs = (f.y & FOLD_SAME) ? same(f.y & GT_OFFSET) : 0.f;
+  return Tsum + rs - M1 - M2;
+}
+
+// One lookup sweep over the hands h0, h0 + hstep, ... < hs: value(record) of
+// every hand to dst, two hands per round, the next round's records requested
+// before this round's values are stored (the stores may alias them, so the
+// compiler would not).
+template <class Rec, class Value>
+__device__ __forceinline__ void lookup_sweep(const Rec* rec, float* dst, int h0, int hstep, int hs, Value value) {
+  Rec a{}, b{};
+  if (h0 < hs) a = rec[h0];
+  if (h0 + hstep < hs) b = rec[h0 + hstep];
+  for (int h = h0; h < hs; h += 2 * hstep) {
+    const Rec ra = a, rb = b;
+    const int h1 = h + hstep, h2 = h1 + hstep, h3 = h2 + hstep;
+    if (h2 < hs) a = rec[h2];
+    b = h3 < hs ? rec[h3] : Rec{};  // past the end: a blocked hand's record, which reads nothing else
+    const float va = value(ra, h), vb = value(rb, h1);
+    dst[h] = va;
+    if (h1 < hs) dst[h1] = vb;
+  }
+}
+
 template <bool GEN, bool SPLIT = false, bool CTA = false>
 __device__ __forceinline__ void warp_terms_inl(const Ctx& c, const Op* ops, int n, int p) {
   static_assert(!CTA || (SPLIT && !GEN), "CTA runs are solve-pass runs of lone spots");
   PHASE_T0(t_scan);
+  extern __shared__ float4 smem4[];
+  float* sm = reinterpret_cast<float*>(smem4);
   const SpotDev& sp = *c.sp;
   const int o = p ^ 1;
-  const int Hp = sp.H[p], hsp = sp.hs[p];
+  const int hsp = sp.hs[p];
   const int lane = threadIdx.x & 31;
   Tables T;
   board_tables(c, ops[0].board, T);
-  const int V = T.nvalid[o], n3 = 3 * V;
-  const uint16_t* g = T.gidx[o];
-  const uint32_t* hd = T.heads[o];
+  const int V = T.nvalid[o];
   const float* rch = slot_in(c, ops[0].src);
-  prefetch_l2_bytes(T.thr[p], 16 * Hp);
   const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   // the scan buffer (in CTA mode warp 0's: buffers are scan_buf_floats apart,
   // one spot a launch); entry j of the gathered list lives at e[j]
   float* buf = shared_view(CTA ? c.buf - (size_t)warp * scan_buf_floats(c.vstride) : c.buf);
   float* e = buf + kScanBase;
-  if (lane == 0 && (!CTA || warp == 0)) st4(buf, make_float4(0.f, 0.f, 0.f, 0.f));  // what empty prefixes read
   // adjoint pass at a depth boundary: the reach is weighted by the payoff
-  // owner's boundary values.  Where the gathered values may be negative
-  // (caller-given reach, boundary weights) segment starts come from the
-  // bitmap; solve passes mark them in the sign bit of the non-negative reach.
+  // owner's boundary values
   const bool adjm = GEN && c.owner >= 0;
   const NodeDev& nd0 = sp.nodes[ops[0].node];
   const float* bw = adjm && ops[0].term == TERM_BOUNDARY
                         ? sp.bcfv + ((size_t)nd0.boundary * 2 + c.owner) * c.vstride
                         : nullptr;
-  const bool bits = GEN && (bw != nullptr || c.signed_reach != 0);
-  {  // 1. gather
-    const int n4 = (n3 + 3) >> 2;  // groups of four entries
-    constexpr int kU = PS_GATHER_U;
-    for (int w0 = (CTA ? warp * 32 * kU : 0) + lane; w0 < n4; w0 += 32 * kU * (CTA ? nwarps : 1)) {
-      uint2 ix[kU];
-      uint32_t hb[kU];
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int w = w0 + 32 * u;
-        ix[u] = w < n4 ? *reinterpret_cast<const uint2*>(g + 4 * w) : make_uint2(0u, 0u);
-        hb[u] = w < n4 ? hd[w >> 3] >> ((4 * w) & 31) : 0u;
-      }
-      float x[kU][4];
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int k = 4 * (w0 + 32 * u);
-        const uint32_t id[4] = {ix[u].x & 0xFFFFu, ix[u].x >> 16, ix[u].y & 0xFFFFu, ix[u].y >> 16};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) x[u][e] = k + e < n3 ? (GEN && bw ? rch[id[e]] * bw[id[e]] : rch[id[e]]) : 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        const int k = 4 * (w0 + 32 * u);
-        if (k >= n3) continue;
-        const uint32_t m = bits ? 0u : hb[u];
-        float4 v;
-        v.x = (m & 1u) ? -x[u][0] : x[u][0];
-        v.y = (m & 2u) ? -x[u][1] : x[u][1];
-        v.z = (m & 4u) ? -x[u][2] : x[u][2];
-        v.w = (m & 8u) ? -x[u][3] : x[u][3];
-        st4(e + k, v);  // entries past n3 are never read
-      }
-    }
-  }
-  if (CTA)
-    __syncthreads();
-  else
-    __syncwarp();
-  if (!CTA || warp == 0) {  // 2. chunked segmented scan
-    const int C = ((n3 + 31) >> 5) | 1;
-    const int lo = min(lane * C, n3), hi = min(lo + C, n3);
+  if (!CTA || warp == 0) {
+    if (lane == 0) st4(buf, make_float4(0.f, 0.f, 0.f, 0.f));  // what empty prefixes and blocked hands read
+    const int C = scan_chunk(3 * V), G = (C + 7) >> 3;
+    const uint4* gt = T.gt[o] + lane;
+    float* el = e + lane * C;
+    const int nf = reinterpret_cast<const uint16_t*>(T.gt[o] + 32 * G)[lane];  // entries before the first start
     float run = 0.f;
-    int first = hi;
-    if (bits) {
-      for (int j = lo; j < hi; ++j) {
-        const float x = e[j];
-        if ((hd[j >> 5] >> (j & 31)) & 1u) {
-          run = x;
-          first = min(first, j);
-        } else {
-          run = __fadd_rn(run, x);
-        }
-        e[j] = run;
+    // 1. gather and scan
+    uint4 w = gt[0];
+    for (int g = 0; g < G; ++g) {
+      const uint32_t wd[4] = {w.x, w.y, w.z, w.w};
+      float x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t off = (u & 1 ? wd[u >> 1] >> 16 : wd[u >> 1]) & GT_OFFSET;
+        x[u] = byte_at(rch, off);
+        if (GEN && bw) x[u] *= byte_at(bw, off);
       }
-    } else {
-      // a segment start carries the sign bit of its non-negative value
-#pragma unroll 2
-      for (int j = lo; j < hi; ++j) {
-        const float x = e[j], y = fabsf(x);
-        run = signbit(x) ? y : __fadd_rn(run, y);
-        e[j] = run;
-      }
-      // the chunk's first segment start, from the bitmap the signs came from
-      for (int w = lo >> 5; lo < hi && w <= (hi - 1) >> 5; ++w) {
-        const uint32_t m = hd[w] & (w == lo >> 5 ? ~0u << (lo & 31) : ~0u);
-        if (m) {
-          first = min(hi, (w << 5) + __ffs(m) - 1);
-          break;
-        }
+      if (g + 1 < G) w = gt[32 * (g + 1)];
+      const int m = C - 8 * g;  // entries of this round: 8, fewer in the last
+      auto add = [&](int u) {
+        const bool head = wd[u >> 1] & (u & 1 ? GT_HEAD << 16 : GT_HEAD);
+        run = head ? x[u] : __fadd_rn(run, x[u]);
+        el[8 * g + u] = run;
+      };
+      if (m >= 8) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) add(u);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 7; ++u)
+          if (u < m) add(u);
       }
     }
+    // 2. carry-ins.  (Entries past the list's end repeat the first reach value;
+    // only sums past the list's end see them.)
     float v = run;
-    bool f = first < hi;
+    bool f = nf < C;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const float vv = __shfl_up_sync(0xffffffffu, v, d);
@@ -565,7 +585,15 @@ __device__ __forceinline__ void warp_terms_inl(const Ctx& c, const Op* ops, int 
     }
     float in = __shfl_up_sync(0xffffffffu, v, 1);
     if (lane == 0) in = 0.f;
-    for (int j = lo; j < first; ++j) e[j] = __fadd_rn(e[j], in);
+    int j = 0;
+    for (; j + 4 <= nf; j += 4) {
+      const float a0 = el[j], a1 = el[j + 1], a2 = el[j + 2], a3 = el[j + 3];
+      el[j] = __fadd_rn(a0, in);
+      el[j + 1] = __fadd_rn(a1, in);
+      el[j + 2] = __fadd_rn(a2, in);
+      el[j + 3] = __fadd_rn(a3, in);
+    }
+    for (; j < nf; ++j) el[j] = __fadd_rn(el[j], in);
   }
   if (CTA)
     __syncthreads();
@@ -578,8 +606,7 @@ __device__ __forceinline__ void warp_terms_inl(const Ctx& c, const Op* ops, int 
     for (int h = lane; h < sp.H[o]; h += 32) row[h] = rch[h];
   }
   // 3. lookups: every prefix is one load at a position of the hand's record
-  const uint4* thr = T.thr[p];
-  const uint16_t* same = sp.same[p];
+  const uint32_t bb = (uint32_t)(buf - sm) * 0x10001u;  // the buffer's position, for both halves of a word
   const float Tsum = buf[kScanBase - 1 + V];  // all V entries (0 when V = 0)
   const int pay = adjm ? c.owner : p;  // whose payoffs the values are
   const int part = CTA ? warp : SPLIT ? c.part : 0, parts = CTA ? nwarps : SPLIT ? c.parts : 1;
@@ -589,106 +616,53 @@ __device__ __forceinline__ void warp_terms_inl(const Ctx& c, const Op* ops, int 
     const NodeDev& nd = sp.nodes[op.node];
     float* dst = slot_at(c, op.dst);
     const float aw = nd.amount_win, al = nd.amount_lose;
-    // showdown coefficients of the traverser's win / loss (swapped when the
-    // values are the opponent's payoffs)
-    const float cw = adjm ? al : aw, cl = adjm ? aw : al;
-    float* grow = GEN && c.bgrad && op.term == TERM_BOUNDARY && !adjm
-                      ? c.bgrad + ((size_t)nd.boundary * 2 + p) * c.vstride
-                      : nullptr;
-    // the next hand's record is requested before this hand's value is stored:
-    // the store may alias it, so the compiler would not issue it earlier
-    uint4 tn = h0 < Hp ? thr[h0] : make_uint4(THR_INVALID, 0, 0, 0);
-    if (!GEN && op.term == TERM_BOUNDARY) {
-      // depth-boundary values in a loop of their own, which keeps the fold /
-      // showdown loop of full trees small (evaluation.rs:544-605)
-      const float* brow = sp.bcfv + ((size_t)nd.boundary * 2 + p) * c.vstride;
-      for (int h = h0; h < hsp; h += hstep) {
-        float v = 0.f;
-        const uint4 t = tn;
-        tn = h + hstep < Hp ? thr[h + hstep] : make_uint4(THR_INVALID, 0, 0, 0);
-        if (t.x != THR_INVALID) {
-          const float M1 = buf[t.z & 0xFFFF], M2 = buf[t.w >> 16];
-          const uint32_t si = same[h];
-          const float rs = si != 0xFFFF ? rch[si] : 0.f;
-          const float adj = Tsum + rs - M1 - M2;
-          v = __fmul_rn(__fmul_rn(brow[h], nd.payoff_scale), adj);
+    if (op.term == TERM_SHOWDOWN) {
+      // showdown coefficients of the traverser's win / loss (swapped when the
+      // values are the opponent's payoffs)
+      const float cw = adjm ? al : aw, cl = adjm ? aw : al;
+      if (!sp.raked) {
+        lookup_sweep(T.thr[p], dst, h0, hstep, hsp,
+                     [&](uint4 t, int) { return showdown_value(sm, bb, t, Tsum, cw, cl); });
+      } else {
+        const uint16_t* same = sp.same[p];
+        const float ctie = nd.amount_tie;
+        for (int h = h0; h < hsp; h += hstep) {
+          const uint4 t = T.thr[p][h];
+          float v = 0.f;
+          if (t.x) {
+            const float Plt = buf[t.x & 0xFFFF], Ple = buf[t.x >> 16];
+            const float Q1lt = buf[t.y & 0xFFFF], Q1le = buf[t.y >> 16];
+            const float M1 = buf[t.z & 0xFFFF], Q2lt = buf[t.z >> 16];
+            const float Q2le = buf[t.w & 0xFFFF], M2 = buf[t.w >> 16];
+            v = raked_showdown_value(cw, cl, ctie, Plt - Q1lt - Q2lt, Ple, Q1le, Q2le, Tsum, M1, M2, rch, same[h]);
+          }
+          dst[h] = v;
         }
-        dst[h] = v;
       }
-      continue;
-    }
-    // whole-warp runs (no split copies: those of the lone-spot grid ran slower so)
-    if (!GEN && !SPLIT && op.term == TERM_SHOWDOWN && !sp.raked) {  // unraked showdowns in a loop of their own
-#pragma unroll 2
-      for (int h = h0; h < hsp; h += hstep) {
-        float v = 0.f;
-        const uint4 t = tn;
-        tn = h + hstep < Hp ? thr[h + hstep] : make_uint4(THR_INVALID, 0, 0, 0);
-        if (t.x != THR_INVALID) {
-          const float M1 = buf[t.z & 0xFFFF], M2 = buf[t.w >> 16];
-          const float Plt = buf[t.x & 0xFFFF], Ple = buf[t.x >> 16];
-          const float Q1lt = buf[t.y & 0xFFFF], Q1le = buf[t.y >> 16];
-          const float Q2lt = buf[t.z >> 16], Q2le = buf[t.w & 0xFFFF];
-          const float win = Plt - Q1lt - Q2lt;
-          const float lose = (Tsum - Ple) - (M1 - Q1le) - (M2 - Q2le);
-          v = __fadd_rn(__fmul_rn(cw, win), __fmul_rn(cl, lose));
-        }
-        dst[h] = v;
-      }
-      continue;
-    }
-    if (!GEN && !SPLIT && op.term == TERM_FOLD) {  // folds in a loop of their own
+    } else if (op.term == TERM_FOLD) {
       const float cf = op.fold_pl != pay ? aw : al;
-#pragma unroll 2
-      for (int h = h0; h < hsp; h += hstep) {
-        float v = 0.f;
-        const uint4 t = tn;
-        tn = h + hstep < Hp ? thr[h + hstep] : make_uint4(THR_INVALID, 0, 0, 0);
-        if (t.x != THR_INVALID) {
-          const float M1 = buf[t.z & 0xFFFF], M2 = buf[t.w >> 16];
-          const uint32_t si = same[h];
-          const float rs = si != 0xFFFF ? rch[si] : 0.f;
-          const float adj = Tsum + rs - M1 - M2;
-          v = __fmul_rn(cf, adj);
-        }
-        dst[h] = v;
-      }
-      continue;
-    }
-    for (int h = h0; h < hsp; h += hstep) {
-      float v = 0.f;
-      const uint4 t = tn;
-      tn = h + hstep < Hp ? thr[h + hstep] : make_uint4(THR_INVALID, 0, 0, 0);
-      if (t.x != THR_INVALID) {
-        const float M1 = buf[t.z & 0xFFFF], M2 = buf[t.w >> 16];
-        if (op.term == TERM_SHOWDOWN) {
-          const float Plt = buf[t.x & 0xFFFF], Ple = buf[t.x >> 16];
-          const float Q1lt = buf[t.y & 0xFFFF], Q1le = buf[t.y >> 16];
-          const float Q2lt = buf[t.z >> 16], Q2le = buf[t.w & 0xFFFF];
-          const float win = Plt - Q1lt - Q2lt;
-          if (!sp.raked) {
-            const float lose = (Tsum - Ple) - (M1 - Q1le) - (M2 - Q2le);
-            v = __fadd_rn(__fmul_rn(cw, win), __fmul_rn(cl, lose));
-          } else {
-            v = raked_showdown_value(cw, cl, nd.amount_tie, win, Ple, Q1le, Q2le, Tsum, M1, M2, rch, same[h]);
-          }
-        } else {
-          const uint32_t si = same[h];
-          const float rs = si != 0xFFFF ? (GEN && bw ? rch[si] * bw[si] : rch[si]) : 0.f;
-          const float adj = Tsum + rs - M1 - M2;
-          if (op.term == TERM_FOLD) {
-            v = __fmul_rn(op.fold_pl != pay ? aw : al, adj);
-          } else if (GEN && adjm) {
-            v = __fmul_rn(nd.payoff_scale, adj);
-          } else if (GEN) {  // boundary values of the general passes (solve passes loop above)
-            const float bv = sp.bcfv[((size_t)nd.boundary * 2 + p) * c.vstride + h];
-            v = __fmul_rn(__fmul_rn(bv, nd.payoff_scale), adj);
-            if (grow) grow[h] = __fmul_rn(nd.payoff_scale, adj);
-          }
-        }
-      }
-      if (GEN && grow && t.x == THR_INVALID) grow[h] = 0.f;
-      dst[h] = v;
+      lookup_sweep(T.fold[p], dst, h0, hstep, hsp, [&](uint2 f, int) {
+        const float v = __fmul_rn(cf, blocked_reach(sm, bb, f, Tsum, [&](uint32_t off) { return byte_at(rch, off); }));
+        return (f.y & FOLD_VALID) ? v : 0.f;
+      });
+    } else if (GEN && adjm) {  // depth boundary, adjoint: the payoff owner's values weight the reach
+      const float scale = nd.payoff_scale;
+      lookup_sweep(T.fold[p], dst, h0, hstep, hsp, [&](uint2 f, int) {
+        const float v = __fmul_rn(scale, blocked_reach(sm, bb, f, Tsum, [&](uint32_t off) {
+                          return bw ? byte_at(rch, off) * byte_at(bw, off) : byte_at(rch, off);
+                        }));
+        return (f.y & FOLD_VALID) ? v : 0.f;
+      });
+    } else {  // depth boundary (evaluation.rs:544-605)
+      const float scale = nd.payoff_scale;
+      const float* brow = sp.bcfv + ((size_t)nd.boundary * 2 + p) * c.vstride;
+      float* grow = GEN && c.bgrad ? c.bgrad + ((size_t)nd.boundary * 2 + p) * c.vstride : nullptr;
+      lookup_sweep(T.fold[p], dst, h0, hstep, hsp, [&](uint2 f, int h) {
+        const float adj = blocked_reach(sm, bb, f, Tsum, [&](uint32_t off) { return byte_at(rch, off); });
+        const bool ok = f.y & FOLD_VALID;
+        if (GEN && grow && h < hsp) grow[h] = ok ? __fmul_rn(scale, adj) : 0.f;
+        return ok ? __fmul_rn(__fmul_rn(brow[h], scale), adj) : 0.f;
+      });
     }
   }
   if (GEN && bw && c.bgrad) {  // dV/dB = (scale * blocked opponent reach) * own adjoint reach / chance path
@@ -1103,28 +1077,26 @@ __device__ bool bind_ctx(Ctx& c, const SpotDev* sp, float* scratch, size_t scrat
     return false;
   }
   for (int q = 0; q < 2; ++q) {
-    c.t0.gidx[q] = sp->gidx[q];
-    c.t0.heads[q] = sp->heads[q];
+    c.t0.gt[q] = reinterpret_cast<const uint4*>(sp->gt[q]);
     c.t0.thr[q] = reinterpret_cast<const uint4*>(sp->thr[q]);
+    c.t0.fold[q] = reinterpret_cast<const uint2*>(sp->fold[q]);
     c.t0.nvalid[q] = sp->nvalid[q][0];
   }
   if (staged) {
     __syncthreads();  // the previous spot's users of the staged tables are done
-    uint4* thr_s = reinterpret_cast<uint4*>(tables);
-    uint32_t* hd_s = reinterpret_cast<uint32_t*>(tables + 16 * (sp->hs[0] + sp->hs[1]));
-    uint16_t* g_s = reinterpret_cast<uint16_t*>(hd_s + head_words16(sp->hs[0]) + head_words16(sp->hs[1]));
+    uint4* to = reinterpret_cast<uint4*>(tables);
     for (int q = 0; q < 2; ++q) {
-      const int hs = sp->hs[q];
-      uint4* ts = thr_s + (q ? sp->hs[0] : 0);
-      const uint4* tg = reinterpret_cast<const uint4*>(sp->thr[q]);
-      for (int i = threadIdx.x; i < hs; i += blockDim.x) ts[i] = tg[i];
-      uint32_t* hs_ = hd_s + (q ? head_words16(sp->hs[0]) : 0);
-      for (int i = threadIdx.x; i < head_words(hs); i += blockDim.x) hs_[i] = sp->heads[q][i];
-      uint16_t* gs = g_s + (q ? 3 * sp->hs[0] : 0);
-      for (int i = threadIdx.x; i < 3 * hs; i += blockDim.x) gs[i] = sp->gidx[q][i];
-      c.t0.thr[q] = ts;
-      c.t0.heads[q] = hs_;
-      c.t0.gidx[q] = gs;
+      const int hs = sp->hs[q], ng = gather_vecs(hs);
+      for (int i = threadIdx.x; i < hs; i += blockDim.x) to[i] = c.t0.thr[q][i];
+      c.t0.thr[q] = to;
+      to += hs;
+      for (int i = threadIdx.x; i < ng; i += blockDim.x) to[i] = c.t0.gt[q][i];
+      c.t0.gt[q] = to;
+      to += ng;
+      const uint4* fs = reinterpret_cast<const uint4*>(c.t0.fold[q]);  // two 8-byte records each (hs is a multiple of 4)
+      for (int i = threadIdx.x; i < hs / 2; i += blockDim.x) to[i] = fs[i];
+      c.t0.fold[q] = reinterpret_cast<const uint2*>(to);
+      to += hs / 2;
     }
     __syncthreads();
   }
@@ -1578,9 +1550,9 @@ __device__ void lane_item(const Lane& L, const FlowArgs& A, int term, int idx, f
   if (mode == M_DCFR && sp.SG != nullptr)
     c.sg = SG_WRITE | (p == 1 || L.t > (A.job.checks ? 0 : A.job.t0) ? SG_READ : 0);
   for (int q = 0; q < 2; ++q) {
-    c.t0.gidx[q] = sp.gidx[q];
-    c.t0.heads[q] = sp.heads[q];
+    c.t0.gt[q] = reinterpret_cast<const uint4*>(sp.gt[q]);
     c.t0.thr[q] = reinterpret_cast<const uint4*>(sp.thr[q]);
+    c.t0.fold[q] = reinterpret_cast<const uint2*>(sp.fold[q]);
     c.t0.nvalid[q] = sp.nvalid[q][0];
   }
   const Discount dc = mode == M_DCFR ? A.disc[L.t] : Discount{0.f, 0.f, 0.f, 0.f};
@@ -1938,6 +1910,7 @@ struct SetupSmem {
   uint16_t coff[2][56];
   uint16_t strength[2][kSetupMaxH];
   int nvalid[2];
+  int first[32];  // per lane: entries of its scan chunk before the first segment start
 };
 
 __global__ void k_setup(const SpotDev* __restrict__ spots, const int2* __restrict__ work, int nwork,
@@ -1989,6 +1962,7 @@ __global__ void k_setup(const SpotDev* __restrict__ spots, const int2* __restric
       }
       __syncthreads();
       const int V = S.nvalid[q];
+      if (threadIdx.x < 32) S.first[threadIdx.x] = scan_chunk(3 * V);
       // card groups: keys (card << 16 | position in strength order)
       for (int i = threadIdx.x; i < kSortN2; i += blockDim.x) {
         uint32_t key = 0xFFFFFFFFu;
@@ -2002,12 +1976,11 @@ __global__ void k_setup(const SpotDev* __restrict__ spots, const int2* __restric
       }
       __syncthreads();
       bitonic_sort_u32(S.keys, kSortN2);
-      uint16_t* gidx = sp.gidx[q] + (size_t)b * 3 * sp.hs[q];
-      for (int i = threadIdx.x; i < V; i += blockDim.x) gidx[i] = S.ord[q][i];
+      uint16_t* ord = sp.ord[q] + (size_t)b * sp.hs[q];
+      for (int i = threadIdx.x; i < V; i += blockDim.x) ord[i] = S.ord[q][i];
       for (int i = threadIdx.x; i < 2 * V; i += blockDim.x) {
         const uint32_t key = S.keys[i];
         const int k = key & 0xFFFF;
-        gidx[V + i] = S.ord[q][k];
         S.istr[q][i] = S.sord[q][k];
         const int card = key >> 16;
         const int prev = i == 0 ? -1 : (int)(S.keys[i - 1] >> 16);
@@ -2016,49 +1989,46 @@ __global__ void k_setup(const SpotDev* __restrict__ spots, const int2* __restric
           for (int cc = card + 1; cc <= 52; ++cc) S.coff[q][cc] = (uint16_t)(2 * V);
       }
       if (V == 0 && threadIdx.x < 53) S.coff[q][threadIdx.x] = 0;
-      __syncthreads();
-      uint16_t* co = sp.coff[q] + (size_t)b * 56;
-      if (threadIdx.x < 56) co[threadIdx.x] = threadIdx.x <= 52 ? S.coff[q][threadIdx.x] : 0;
       if (threadIdx.x == 0) sp.nvalid[q][b] = V;
-      // segment starts of the gather list: 0 (strength order) and every non-empty card group
-      uint32_t* hd = sp.heads[q] + (size_t)b * head_words(sp.hs[q]);
-      for (int i = threadIdx.x; i < head_words(sp.hs[q]); i += blockDim.x) {
-        uint32_t wv = 0;
-        for (int bit = 0; bit < 32; ++bit) {
-          const int k = 32 * i + bit;
-          bool h = k == 0 && V > 0;
-          if (k >= V && k < 3 * V) {
-            const int r = k - V;
-            // r starts a group if it equals coff[c] for a non-empty group c
-            int lo = 0, hi = 52;
-            while (lo < hi) {
-              const int m = (lo + hi) >> 1;
-              if (S.coff[q][m + 1] <= r) lo = m + 1;
-              else hi = m;
-            }
-            h = S.coff[q][lo] == r;
-          }
-          if (h) wv |= 1u << bit;
+      // gather table: entry j of lane l's chunk is entry l C + j of the list
+      // (the V hands in strength order, then every card's hands), a segment
+      // start at 0 and at every card group; eight entries of a lane together
+      const int n3 = 3 * V, C = scan_chunk(n3), G = (C + 7) >> 3;
+      uint16_t* gt = sp.gt[q] + (size_t)b * 8 * gather_vecs(sp.hs[q]);
+      for (int i = threadIdx.x; i < 256 * G; i += blockDim.x) {
+        const int j = (i >> 8) * 8 + (i & 7), k = ((i >> 3) & 31) * C + j;
+        uint32_t x = 0;  // past the chunk or the list
+        if (j < C && k < n3) {
+          const int r = k - V;
+          const int h = r < 0 ? S.ord[q][k] : S.ord[q][S.keys[r] & 0xFFFF];
+          const bool head = r < 0 ? k == 0 : r == 0 || (S.keys[r] >> 16) != (S.keys[r - 1] >> 16);
+          x = (uint32_t)h * 4 | (head ? GT_HEAD : 0u);
+          if (head) atomicMin(&S.first[(i >> 3) & 31], j);
         }
-        hd[i] = wv;
+        gt[i] = (uint16_t)x;
       }
       __syncthreads();
+      if (threadIdx.x < 32) gt[256 * G + threadIdx.x] = (uint16_t)S.first[threadIdx.x];
     }
     // lookup records of player p's hands against opponent o = p ^ 1, 16 bytes per
     // hand: the scan-buffer positions of the hand's eight prefixes (see the
-    // terminal evaluation above); x = ~0 if the hand is blocked on this board.
+    // terminal evaluation above), all zero if the hand is blocked on this board.
     // With lt / le the opponent hands strictly weaker / weaker-or-tied and l / e
     // the same counts inside card group c (starting at a_c, n_c entries):
     //   P(k)    = kScanBase - 1 + k           (k = 0 reads the zero below the list)
     //   Q_c(k)  = k ? kScanBase - 1 + V + a_c + k : 0
     //   x = P(lt) | P(le) << 16, y = Q_c1(l1) | Q_c1(e1) << 16,
     //   z = Q_c1(n_c1) | Q_c2(l2) << 16, w = Q_c2(e2) | Q_c2(n_c2) << 16
+    // and the 8-byte fold records: x = Q_c1(n_c1) | Q_c2(n_c2) << 16, y = FOLD_VALID and, if the
+    // opponent's list has the same hand, FOLD_SAME | the byte offset of its reach value
     for (int p = 0; p < 2; ++p) {
       const int o = p ^ 1;
       const int Hp = sp.H[p], hsp = sp.hs[p], Vo = S.nvalid[o];
       uint4* thr = reinterpret_cast<uint4*>(sp.thr[p]) + (size_t)b * hsp;
+      uint2* fold = reinterpret_cast<uint2*>(sp.fold[p]) + (size_t)b * hsp;
       for (int h = threadIdx.x; h < hsp; h += blockDim.x) {
-        uint4 v = make_uint4(THR_INVALID, 0, 0, 0);
+        uint4 v = make_uint4(0, 0, 0, 0);
+        uint2 fv = make_uint2(0, 0);
         if (h < Hp) {
           const int c1 = sp.cards[p][2 * h], c2 = sp.cards[p][2 * h + 1];
           const bool ok = !((bmask >> c1) & 1) && !((bmask >> c2) & 1);
@@ -2075,9 +2045,13 @@ __global__ void k_setup(const SpotDev* __restrict__ spots, const int2* __restric
             v.y = Q(a1, l1) | (Q(a1, e1) << 16);
             v.z = Q(a1, (uint32_t)n1) | (Q(a2, l2) << 16);
             v.w = Q(a2, e2) | (Q(a2, (uint32_t)n2) << 16);
+            const uint32_t si = sp.same[p][h];
+            fv.x = (v.z & 0xFFFFu) | (v.w & 0xFFFF0000u);
+            fv.y = FOLD_VALID | (si != 0xFFFF ? FOLD_SAME | 4 * si : 0u);
           }
         }
         thr[h] = v;
+        fold[h] = fv;
       }
     }
     __syncthreads();

@@ -8,21 +8,25 @@
 
 namespace ps {
 
-__host__ __device__ inline int head_words(int hs) { return (3 * hs + 31) / 32; }
-// bitmap words rounded up to 16 bytes, so staged gather lists stay 16-byte aligned
-__host__ __device__ inline int head_words16(int hs) { return (head_words(hs) + 3) & ~3; }
+// The scan of a terminal's 3V-entry list: lane l takes entries [l C, (l + 1) C)
+// with an odd C, so the lanes' strided shared-memory accesses fall in distinct
+// banks.
+__host__ __device__ inline int scan_chunk(int n3) { return ((n3 + 31) >> 5) | 1; }
+// 16-byte vectors of one board's gather table for up to hs hands: eight u16
+// entries per lane and round, then a u16 per lane (entries before the chunk's
+// first segment start).
+__host__ __device__ inline int gather_vecs(int hs) { return 32 * ((scan_chunk(3 * hs) + 7) >> 3) + 4; }
 
 // Board tables of one board staged in shared memory: lookup records (16 bytes
-// per hand), segment-start bitmaps and gather lists (u16, 3 * hs per player).
+// per hand), gather tables and fold records (8 bytes per hand).
 __host__ __device__ inline int table_bytes_for(int hs0, int hs1) {
-  int b = 16 * (hs0 + hs1) + 4 * (head_words16(hs0) + head_words16(hs1)) + 2 * (3 * hs0 + 3 * hs1);
-  return (b + 15) & ~15;
+  return 24 * (hs0 + hs1) + 16 * (gather_vecs(hs0) + gather_vecs(hs1));
 }
 
 // A terminal scan buffer: four zero floats (what an empty prefix reads), then
-// the 3V entries of the gathered list, rounded up to whole float4s.
+// the 32 chunks of the gathered list.
 constexpr int kScanBase = 4;
-__host__ __device__ inline int scan_buf_floats(int vstride) { return 3 * vstride + 2 * kScanBase; }
+__host__ __device__ inline int scan_buf_floats(int vstride) { return kScanBase + 32 * scan_chunk(3 * vstride); }
 
 // Shared-memory plan of one solve CTA (computed on the host per launch): one
 // terminal scan buffer (scan_buf_floats(vstride) floats) per scan warp,
