@@ -196,10 +196,16 @@ int ps_boundary_reach(ps_game* g, float* out);
  *   reach [n][2][1326]      OOP and IP reach at the boundary, combo order
  *   hands [H]               combo index of each output hand
  *   out   [n][2][H]         player 0 averaged with IP-reach weights, player 1 with OOP
- * stream: a cudaStream_t (NULL = the default stream); returns after the work is done. */
+ * stream: a cudaStream_t (NULL = the default stream, never one that is being
+ * captured into a graph); returns after the work is done. */
 int ps_boundary_river_reduce(int32_t n, const uint8_t* boards, const float* pots, const float* stacks,
                              const void* net, int32_t net_bf16, const float* reach, const int32_t* hands, int32_t H,
                              float* out, void* stream);
+/* The gradient of that average with respect to the network outputs, for every
+ * combo in order (H = 1326) and a scale per item (host [n], pot + stack in the
+ * average): g [n][2][1326] -> gy [n][2][48][1326], f32 device arrays. */
+int ps_river_average_grad(int32_t n, const uint8_t* boards, const float* scale, const float* reach, const float* g,
+                          float* gy, void* stream);
 /* The first Linear layer (h outputs over the 2720 inputs) of a boundary
  * network for every input row that ps_boundary_encode would write, without
  * writing those rows (no reference counterpart; the reference runs the layer

@@ -1588,6 +1588,45 @@ std::vector<float> normalized_strategy(ps_game* G, const ArenaNode& n) {  // uti
 }
 }  // namespace
 
+// The datagen entry points check their boards on the host, pass the items'
+// metadata with each launch (kMetaItems at a time) and return when their work
+// is done.  They are not recorded into a graph: the metadata is the caller's
+// host memory at the time of the call.
+static int item_boards(int32_t n, const uint8_t* boards) {
+  for (int i = 0; i < n; ++i) {
+    uint64_t seen = 0;
+    for (int k = 0; k < 4; ++k) {
+      const uint8_t c = boards[4 * i + k];
+      if (c >= 52 || (seen >> c & 1)) return fail(PS_ERR_INVALID, "boards must hold 4 distinct cards below 52");
+      seen |= 1ull << c;
+    }
+  }
+  return PS_OK;
+}
+
+// launch(first item, items, meta) over chunks of the items; meta.a and meta.b
+// from a(i) and b(i)
+template <class A, class B, class Launch>
+static int for_items(int32_t n, const uint8_t* boards, cudaStream_t s, A a, B b, Launch launch) {
+  int rc = item_boards(n, boards);
+  if (rc) return rc;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CU(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return fail(PS_ERR_CUDA, "the datagen kernels cannot be captured into a graph");
+  ItemMeta m;
+  for (int i0 = 0; i0 < n; i0 += kMetaItems) {
+    const int k = std::min(n - i0, kMetaItems);
+    std::memcpy(m.board, boards + 4 * (size_t)i0, 4 * (size_t)k);
+    for (int i = 0; i < k; ++i) {
+      m.a[i] = a(i0 + i);
+      m.b[i] = b(i0 + i);
+    }
+    CU(launch(i0, k, m));
+  }
+  CU(cudaStreamSynchronize(s));
+  return PS_OK;
+}
+
 extern "C" {
 
 const char* ps_last_error(void) { return g_err.c_str(); }
@@ -1908,30 +1947,27 @@ int ps_boundary_river_reduce(int32_t n, const uint8_t* boards, const float* pots
   if (n < 0 || H < 0 || H > 1326 || (n > 0 && (!boards || !pots || !stacks || !net || !reach || !hands || !out)))
     return fail(PS_ERR_INVALID, "bad argument");
   if (n == 0 || H == 0) return PS_OK;
-  std::vector<uint8_t> hb((size_t)n * 4);
-  std::vector<float> dn(n);
-  for (int i = 0; i < n; ++i) {
-    uint64_t seen = 0;
-    for (int k = 0; k < 4; ++k) {
-      const uint8_t c = boards[4 * i + k];
-      if (c >= 52 || (seen >> c & 1)) return fail(PS_ERR_INVALID, "boards must hold 4 distinct cards below 52");
-      seen |= 1ull << c;
-      hb[4 * i + k] = c;
-    }
-    dn[i] = (float)((double)pots[i] + (double)stacks[i]);
-  }
-  cudaStream_t s = (cudaStream_t)stream;
-  StagingLease lease;
-  CU(lease.acquire(hb.size() + 4 * dn.size() + 16));
-  lease.using_stream(s);
-  char* d = lease.ptr;
-  float* d_dn = (float*)(d + ((hb.size() + 15) & ~(size_t)15));
-  CU(cudaMemcpyAsync(d, hb.data(), hb.size(), cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(d_dn, dn.data(), 4 * dn.size(), cudaMemcpyHostToDevice, s));
-  CU(launch_boundary_river_reduce(n, (const uint8_t*)d, d_dn, net, net_bf16 ? 1 : 0, reach, hands, H, out, s));
-  CU(cudaStreamSynchronize(s));
-  lease.done();
-  return PS_OK;
+  const size_t row = (size_t)2 * 48 * 1326 * (net_bf16 ? 2 : 4);
+  return for_items(
+      n, boards, (cudaStream_t)stream, [&](int i) { return (float)((double)pots[i] + (double)stacks[i]); },
+      [](int) { return 0.f; },
+      [&](int i0, int k, const ItemMeta& m) {
+        return launch_boundary_river_reduce(k, m, (const char*)net + i0 * row, net_bf16 ? 1 : 0,
+                                            reach + (size_t)i0 * 2652, hands, H, out + (size_t)i0 * 2 * H,
+                                            (cudaStream_t)stream);
+      });
+}
+
+int ps_river_average_grad(int32_t n, const uint8_t* boards, const float* scale, const float* reach, const float* g,
+                          float* gy, void* stream) {
+  if (n < 0 || (n > 0 && (!boards || !scale || !reach || !g || !gy))) return fail(PS_ERR_INVALID, "bad argument");
+  if (n == 0) return PS_OK;
+  return for_items(
+      n, boards, (cudaStream_t)stream, [&](int i) { return scale[i]; }, [](int) { return 0.f; },
+      [&](int i0, int k, const ItemMeta& m) {
+        return launch_river_average_grad(k, m, reach + (size_t)i0 * 2652, g + (size_t)i0 * 2652,
+                                         gy + (size_t)i0 * 2 * 48 * 1326, (cudaStream_t)stream);
+      });
 }
 
 int ps_boundary_first_layer(int32_t n, const uint8_t* boards, const float* pots, const float* stacks,
@@ -2755,31 +2791,15 @@ int ps_boundary_encode(int32_t n, const uint8_t* boards, const float* pots, cons
   if (n < 0 || (n > 0 && (!boards || !pots || !stacks || !reach || !out)))
     return fail(PS_ERR_INVALID, "bad argument");
   if (n == 0) return PS_OK;
-  std::vector<uint8_t> hb((size_t)n * 4);
-  for (int i = 0; i < n; ++i) {
-    uint64_t seen = 0;
-    for (int k = 0; k < 4; ++k) {
-      const uint8_t c = boards[4 * i + k];
-      if (c >= 52 || (seen >> c & 1)) return fail(PS_ERR_INVALID, "boards must hold 4 distinct cards below 52");
-      seen |= 1ull << c;
-      hb[4 * i + k] = c;
-    }
-  }
-  cudaStream_t s = (cudaStream_t)stream;
-  const size_t ob = ((hb.size() + 15) & ~(size_t)15);
-  StagingLease lease;
-  CU(lease.acquire(ob + 8 * (size_t)n + 16));
-  lease.using_stream(s);
-  char* d = lease.ptr;
-  float* d_pot = (float*)(d + ob);
-  float* d_stack = d_pot + n;
-  CU(cudaMemcpyAsync(d, hb.data(), hb.size(), cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(d_pot, pots, 4 * (size_t)n, cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(d_stack, stacks, 4 * (size_t)n, cudaMemcpyHostToDevice, s));
-  CU(launch_boundary_encode(n, (const uint8_t*)d, d_pot, d_stack, reach, out, out_bf16 ? 1 : 0, s));
-  CU(cudaStreamSynchronize(s));
-  lease.done();
-  return PS_OK;
+  if (((uintptr_t)out & (out_bf16 ? 7 : 15)) != 0)
+    return fail(PS_ERR_INVALID, "out must be aligned to 16 bytes (8 for bf16)");
+  const size_t row = (size_t)2 * 48 * kBoundaryInput * (out_bf16 ? 2 : 4);
+  return for_items(
+      n, boards, (cudaStream_t)stream, [&](int i) { return pots[i]; }, [&](int i) { return stacks[i]; },
+      [&](int i0, int k, const ItemMeta& m) {
+        return launch_boundary_encode(k, m, reach + (size_t)i0 * 2652, (char*)out + i0 * row, out_bf16 ? 1 : 0,
+                                      (cudaStream_t)stream);
+      });
 }
 
 int ps_batch_results(ps_batch* pb, float* expl, int32_t* iters) {

@@ -21,83 +21,184 @@ constexpr int kRivers = 48;
 constexpr int kCombos = 1326;
 
 // (c1, c2), c1 < c2, of a combo index (inverse of card.rs:50-55): c1 is the
-// last card whose first combo, c1 * (101 - c1) / 2 + c1, is at most idx
+// last card whose first combo, c1 * (103 - c1) / 2, is at most idx
 __device__ __forceinline__ void combo_cards(int idx, int& c1, int& c2) {
-  int a = 0;
-  while (a + 1 < 51 && (a + 1) * (101 - (a + 1)) / 2 + (a + 1) <= idx) ++a;
+  int a = (int)((103.f - sqrtf((float)(10609 - 8 * idx))) * 0.5f);
+  if (a * (103 - a) / 2 > idx) --a;
+  if ((a + 1) * (102 - a) / 2 <= idx) ++a;
   c1 = a;
   c2 = idx - a * (101 - a) / 2 + 1;
 }
-
-__device__ __forceinline__ double net_value(const float* p, size_t i) { return (double)p[i]; }
-__device__ __forceinline__ double net_value(const __nv_bfloat16* p, size_t i) { return (double)__bfloat162float(p[i]); }
-
-template <typename T>
-__global__ void k_boundary_river_reduce(int n, const uint8_t* __restrict__ boards, const float* __restrict__ denorm,
-                                        const T* __restrict__ net, const float* __restrict__ reach,
-                                        const int32_t* __restrict__ hands, int H, float* __restrict__ out) {
-  const int item = blockIdx.x >> 1, p = blockIdx.x & 1, o = p ^ 1;
-  if (item >= n) return;
-  __shared__ double s_w[kRivers];
-  __shared__ double s_red[32];
-  __shared__ uint8_t s_river[kRivers];
-  const uint8_t* bd = boards + 4 * item;
-  if (threadIdx.x == 0) {
-    int k = 0;
-    for (int c = 0; c < 52; ++c)
-      if (c != bd[0] && c != bd[1] && c != bd[2] && c != bd[3]) s_river[k++] = (uint8_t)c;
-  }
-  // total opponent reach
-  const float* ro = reach + ((size_t)item * 2 + o) * kCombos;
-  double t = 0.0;
-  for (int c = threadIdx.x; c < kCombos; c += blockDim.x) t += (double)ro[c];
-  for (int s = 16; s > 0; s >>= 1) t += __shfl_down_sync(0xffffffffu, t, s);
-  if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = t;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tot = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += s_red[w];
-    s_red[0] = tot;
-  }
-  __syncthreads();
-  const double total = s_red[0];
-  // per river: total minus the reach of the 51 combos holding the river card
-  for (int ri = threadIdx.x; ri < kRivers; ri += blockDim.x) {
-    const int r = s_river[ri];
-    double blocked = 0.0;
-    for (int x = 0; x < 52; ++x) {
-      if (x == r) continue;
-      const int a = x < r ? x : r, b = x < r ? r : x;
-      blocked += (double)ro[a * (101 - a) / 2 + b - 1];
-    }
-    s_w[ri] = total - blocked;
-  }
-  __syncthreads();
-  const T* np_ = net + ((size_t)item * 2 + p) * kRivers * kCombos;
-  const double scale = (double)denorm[item];
-  for (int h = threadIdx.x; h < H; h += blockDim.x) {
-    const int combo = hands[h];
-    if (combo < 0 || combo >= kCombos) {  // not a combo: no value
-      out[((size_t)item * 2 + p) * H + h] = 0.0f;
-      continue;
-    }
-    int c1, c2;
-    combo_cards(combo, c1, c2);
-    double num = 0.0, den = 0.0;
-    for (int ri = 0; ri < kRivers; ++ri) {
-      const int r = s_river[ri];
-      if (r == c1 || r == c2) continue;
-      num += s_w[ri] * net_value(np_, (size_t)ri * kCombos + combo);
-      den += s_w[ri];
-    }
-    out[((size_t)item * 2 + p) * H + h] = den > 0.0 ? (float)(num / den * scale) : 0.0f;
-  }
-}
-
 // combo index of two distinct cards (card.rs:50-55)
 __device__ __forceinline__ int combo_index(int a, int b) {
   const int lo = a < b ? a : b, hi = a < b ? b : a;
   return lo * (101 - lo) / 2 + hi - 1;
+}
+
+// The 48 cards not on a 4-card board, ascending; pos: the place of card c in
+// that order (kRivers if it is on the board).
+__device__ __forceinline__ int river_pos(const uint8_t* bd, int c) {
+  int k = c;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (bd[i] == c) return kRivers;
+    k -= bd[i] < c;
+  }
+  return k;
+}
+
+// f64 weight of every river for one item and player: the opponent's reach on
+// the combos free of the river card (total minus the 51 combos holding it).
+// Whole block; s_w [kRivers], s_red [32] shared; ends with a barrier.
+__device__ void river_weights(const uint8_t* bd, const float* ro, double* s_w, double* s_red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double t = 0.0;
+  for (int c = threadIdx.x; c < kCombos; c += blockDim.x) t += (double)ro[c];
+  for (int s = 16; s > 0; s >>= 1) t += __shfl_down_sync(0xffffffffu, t, s);
+  if (lane == 0) s_red[warp] = t;
+  __syncthreads();
+  double total = 0.0;
+  for (int w = 0; w < nw; ++w) total += s_red[w];
+  for (int c = warp; c < 52; c += nw) {  // a warp per card
+    const int k = river_pos(bd, c);
+    if (k == kRivers) continue;
+    double blocked = 0.0;
+    for (int x = lane; x < 52; x += 32)
+      if (x != c) blocked += (double)ro[combo_index(x, c)];
+    for (int s = 16; s > 0; s >>= 1) blocked += __shfl_down_sync(0xffffffffu, blocked, s);
+    if (lane == 0) s_w[k] = total - blocked;
+  }
+  __syncthreads();
+}
+
+// Two adjacent network outputs (an even first index, so the pair is aligned).
+__device__ __forceinline__ float2 net_pair(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 net_pair(const __nv_bfloat16* p) {
+  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+}
+__device__ __forceinline__ float net_one(const float* p) { return *p; }
+__device__ __forceinline__ float net_one(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+
+// One block per (item, player), two hands per thread and round (224 threads:
+// three rounds cover the 663 pairs with 9 idle slots): bound by the read of the
+// network's outputs, the f64 conversions close behind.  The 48 rows of a column
+// pair are read sixteen at a time; whether a river blocks a hand is a bit of a
+// mask, so no branch stands around a load.  One value at a time behind such a
+// branch, 1024 items took 122 us of kernel time for 260 MB of bf16 outputs
+// instead of 99.
+constexpr int kReduceThreads = 224;
+__device__ __forceinline__ uint64_t blocked_rivers(const uint8_t* bd, int combo) {
+  int c1, c2;
+  combo_cards(combo, c1, c2);
+  const int k1 = river_pos(bd, c1), k2 = river_pos(bd, c2);
+  return (1ull << k1 | 1ull << k2) & ((1ull << kRivers) - 1);  // (kRivers: the card is on the board)
+}
+// The sum of the weights of the rivers that do not block a hand: the sum of all
+// less the blocked ones (at most two), added up directly where the difference
+// would cancel.
+__device__ __forceinline__ double free_weight(const double* s_w, double all, uint64_t blocked) {
+  double d = all;
+  for (uint64_t m = blocked; m; m &= m - 1) d -= s_w[__ffsll((long long)m) - 1];
+  if (d > 1e-3 * all) return d;
+  d = 0.0;
+#pragma unroll 1
+  for (int r = 0; r < kRivers; ++r)
+    if (!(blocked >> r & 1)) d += s_w[r];
+  return d;
+}
+__device__ __forceinline__ double all_weights(const double* s_w) {
+  double d = 0.0;
+#pragma unroll 8
+  for (int r = 0; r < kRivers; ++r) d += s_w[r];
+  return d;
+}
+template <typename T>
+__global__ void __launch_bounds__(kReduceThreads) k_boundary_river_reduce(const __grid_constant__ ItemMeta meta,
+                                                                          const T* __restrict__ net,
+                                                                          const float* __restrict__ reach,
+                                                                          const int32_t* __restrict__ hands, int H,
+                                                                          float* __restrict__ out, bool pairs) {
+  const int item = blockIdx.x >> 1, p = blockIdx.x & 1, o = p ^ 1;
+  __shared__ double s_w[kRivers];
+  __shared__ double s_red[32];
+  const uint8_t* bd = meta.board[item];
+  river_weights(bd, reach + ((size_t)item * 2 + o) * kCombos, s_w, s_red);
+  const T* np_ = net + ((size_t)item * 2 + p) * kRivers * kCombos;
+  const double scale = (double)meta.a[item], all = all_weights(s_w);
+  float* dst = out + ((size_t)item * 2 + p) * H;
+  for (int h = 2 * threadIdx.x; h < H; h += 2 * blockDim.x) {
+    const bool two = h + 1 < H;
+    const int ca = hands[h], cb = two ? hands[h + 1] : -1;
+    const bool oka = ca >= 0 && ca < kCombos, okb = cb >= 0 && cb < kCombos;  // not a combo: no value
+    const uint64_t ma = blocked_rivers(bd, oka ? ca : 0), mb = blocked_rivers(bd, okb ? cb : 0);
+    const bool pair = pairs && oka && cb == ca + 1 && !(ca & 1);  // pairs: the outputs are aligned to two values
+    const T* pa = np_ + (oka ? ca : 0);
+    const T* pb = np_ + (okb ? cb : 0);
+    double na = 0.0, nb = 0.0;
+    constexpr int kRows = 16;
+#pragma unroll 1
+    for (int r0 = 0; r0 < kRivers; r0 += kRows) {
+      float2 v[kRows];
+      if (pair) {
+#pragma unroll
+        for (int u = 0; u < kRows; ++u) v[u] = net_pair(pa + (size_t)(r0 + u) * kCombos);
+      } else {
+#pragma unroll
+        for (int u = 0; u < kRows; ++u)
+          v[u] = make_float2(net_one(pa + (size_t)(r0 + u) * kCombos), net_one(pb + (size_t)(r0 + u) * kCombos));
+      }
+      const unsigned ka = (unsigned)(ma >> r0), kb = (unsigned)(mb >> r0);
+#pragma unroll
+      for (int u = 0; u < kRows; ++u) {
+        const double w = s_w[r0 + u];
+        if (!(ka >> u & 1)) na += w * (double)v[u].x;
+        if (!(kb >> u & 1)) nb += w * (double)v[u].y;
+      }
+    }
+    const double da = free_weight(s_w, all, ma), db = free_weight(s_w, all, mb);
+    dst[h] = oka && da > 0.0 ? (float)(na / da * scale) : 0.0f;
+    if (two) dst[h + 1] = okb && db > 0.0 ? (float)(nb / db * scale) : 0.0f;
+  }
+}
+
+// The average's gradient with respect to the network's outputs, in f64 from
+// f32 inputs: gy[i][p][r][c] = w[r] * (g[i][p][c] * scale / sum of w over the
+// rivers free of c's cards), 0 where the river is one of them.  One block per
+// (item, player), a column pair per thread and round: bound by the write of
+// gy.
+__global__ void __launch_bounds__(kReduceThreads) k_river_average_grad(const __grid_constant__ ItemMeta meta,
+                                                            const float* __restrict__ reach,
+                                                            const float* __restrict__ g, float* __restrict__ gy,
+                                                            bool pairs) {
+  const int item = blockIdx.x >> 1, p = blockIdx.x & 1, o = p ^ 1;
+  __shared__ double s_w[kRivers];
+  __shared__ double s_red[32];
+  const uint8_t* bd = meta.board[item];
+  river_weights(bd, reach + ((size_t)item * 2 + o) * kCombos, s_w, s_red);
+  const double scale = (double)meta.a[item], all = all_weights(s_w);
+  const float* gi = g + ((size_t)item * 2 + p) * kCombos;
+  float* go = gy + ((size_t)item * 2 + p) * kRivers * kCombos;
+  for (int c = 2 * threadIdx.x; c < kCombos; c += 2 * blockDim.x) {  // kCombos is even
+    const uint64_t ma = blocked_rivers(bd, c), mb = blocked_rivers(bd, c + 1);
+    const double da = free_weight(s_w, all, ma), db = free_weight(s_w, all, mb);
+    const double ka = da > 0.0 ? (double)gi[c] * scale / da : 0.0, kb = db > 0.0 ? (double)gi[c + 1] * scale / db : 0.0;
+#pragma unroll 1
+    for (int r0 = 0; r0 < kRivers; r0 += 8) {
+      const unsigned xa = (unsigned)(ma >> r0), xb = (unsigned)(mb >> r0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const double w = s_w[r0 + u];
+        const float2 v = make_float2(xa >> u & 1 ? 0.f : (float)(w * ka), xb >> u & 1 ? 0.f : (float)(w * kb));
+        float* at = go + (size_t)(r0 + u) * kCombos + c;
+        if (pairs) {  // gy is aligned to two values
+          *reinterpret_cast<float2*>(at) = v;
+        } else {
+          at[0] = v.x;
+          at[1] = v.y;
+        }
+      }
+    }
+  }
 }
 
 // One block per boundary item (spot, ordinal), both players: between the
@@ -167,81 +268,112 @@ cudaError_t launch_spot_combo(const SpotDev* spots, int n, int which, const floa
   return cudaGetLastError();
 }
 
-// Input rows of the boundary network, one block per (item, player): the
-// item's two reach rows are staged in shared memory and written out once per
-// river card with the hands holding that card zeroed.  Pure store bandwidth:
-// 2720 values per row, written as 16-byte (f32) or 8-byte (bf16) vectors.
+// Input rows of the boundary network, one block per item: bound by the write
+// of the rows.  A thread owns one 16-byte vector of the row (4 f32 or 8 bf16
+// values) for all 48 rivers and both players: it keeps the vector's reach
+// values converted and their hands' cards in registers, and per river only
+// clears the hands holding the river card and stores the vector twice.
+// Choosing each value of each row by its segment, 733 items took 202 us for
+// 383 MB of bf16 rows instead of 91.  The vectors that reach into the 68
+// board, rank, pot, stack and player columns are made value by value, their
+// rows spread over the block.
+constexpr int kEncodeThreads = 352;
 template <bool BF16>
-__global__ void k_boundary_encode(const uint8_t* __restrict__ boards, const float* __restrict__ pots,
-                                  const float* __restrict__ stacks, const float* __restrict__ reach,
-                                  void* __restrict__ out) {
-  const int item = blockIdx.x >> 1, player = blockIdx.x & 1;
-  __shared__ float s_r[2 * kCombos];
-  __shared__ uint16_t s_pair[kCombos];  // c1 | c2 << 8
+__global__ void __launch_bounds__(kEncodeThreads) k_boundary_encode(const __grid_constant__ ItemMeta meta,
+                                                                    const float* __restrict__ reach,
+                                                                    void* __restrict__ out, bool whole) {
+  constexpr int E = BF16 ? 8 : 4;  // values per vector
+  constexpr int kVec = kBoundaryInput / E, kPlain = 2 * kCombos / E;
+  const int item = blockIdx.x;
   __shared__ uint8_t s_river[kRivers];
-  const uint8_t* bd = boards + 4 * item;
-  const uint64_t bmask = (1ull << bd[0]) | (1ull << bd[1]) | (1ull << bd[2]) | (1ull << bd[3]);
-  if (threadIdx.x == 0) {
-    int k = 0;
-    for (int c = 0; c < 52; ++c)
-      if (!(bmask >> c & 1)) s_river[k++] = (uint8_t)c;
+  const uint8_t* bd = meta.board[item];
+  for (int c = threadIdx.x; c < 52; c += blockDim.x) {
+    const int k = river_pos(bd, c);
+    if (k < kRivers) s_river[k] = (uint8_t)c;
   }
-  for (int c1 = threadIdx.x; c1 < 51; c1 += blockDim.x)
-    for (int c2 = c1 + 1; c2 < 52; ++c2) s_pair[combo_index(c1, c2)] = (uint16_t)(c1 | c2 << 8);
-  const float* r = reach + (size_t)item * 2 * kCombos;
-  for (int c = threadIdx.x; c < 2 * kCombos; c += blockDim.x) s_r[c] = r[c];
+  const uint64_t bmask = (1ull << bd[0]) | (1ull << bd[1]) | (1ull << bd[2]) | (1ull << bd[3]);
+  const float* rr = reach + (size_t)item * 2 * kCombos;
   // boundary_evaluator.rs:35-36, :54-56 in f32
-  const float pot = pots[item], stack = stacks[item];
+  const float pot = meta.a[item], stack = meta.b[item];
   const float total = __fadd_rn(pot, stack);
   const float norm = total > 0.f ? total : 1.f;
-  const float fpot = __fdiv_rn(pot, norm), fstack = __fdiv_rn(stack, norm), fpl = (float)player;
+  const float fpot = __fdiv_rn(pot, norm), fstack = __fdiv_rn(stack, norm);
   const unsigned ranks4 = (1u << (bd[0] >> 2)) | (1u << (bd[1] >> 2)) | (1u << (bd[2] >> 2)) | (1u << (bd[3] >> 2));
+  uint4* o0 = reinterpret_cast<uint4*>(out) + (size_t)item * 2 * kRivers * kVec;
+  uint4* o1 = o0 + (size_t)kRivers * kVec;
+  auto bits = [](float x) {
+    return BF16 ? (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x)) : __float_as_uint(x);
+  };
+  auto put = [&](uint4* at, uint4 w) {
+    if (!BF16 || whole) {
+      *at = w;
+    } else {  // bf16 rows aligned to 8 bytes only
+      reinterpret_cast<uint2*>(at)[0] = make_uint2(w.x, w.y);
+      reinterpret_cast<uint2*>(at)[1] = make_uint2(w.z, w.w);
+    }
+  };
+  auto pack = [](const uint32_t (&x)[E]) {
+    return BF16 ? make_uint4(x[0] | x[1] << 16, x[2 % E] | x[3 % E] << 16, x[4 % E] | x[5 % E] << 16,
+                             x[6 % E] | x[7 % E] << 16)
+                : make_uint4(x[0], x[1], x[2], x[3]);
+  };
   __syncthreads();
-  constexpr int kVec = kBoundaryInput / 4;
-  for (int ri = 0; ri < kRivers; ++ri) {
-    const int river = s_river[ri];
+  // the vectors that hold board, rank, pot, stack and player columns
+  constexpr int kTail = kVec - kPlain;
+  for (int i = threadIdx.x; i < 2 * kRivers * kTail; i += blockDim.x) {
+    const int ri = i / kTail, q = kPlain + i - ri * kTail;
+    const int player = ri >= kRivers, river = s_river[player ? ri - kRivers : ri];
     const uint64_t b5 = bmask | (1ull << river);
     const unsigned ranks = ranks4 | (1u << (river >> 2));
-    const size_t row = ((size_t)blockIdx.x * kRivers + ri) * kBoundaryInput;
-    for (int q = threadIdx.x; q < kVec; q += blockDim.x) {
-      float v[4];
+    uint32_t x[E];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int f = 4 * q + e;
-        float x;
-        if (f < 2 * kCombos) {
-          const int c = f < kCombos ? f : f - kCombos;
-          const unsigned pr = s_pair[c];
-          x = ((pr & 0xFF) == (unsigned)river || (pr >> 8) == (unsigned)river) ? 0.f : s_r[f];
-        } else if (f < 2 * kCombos + 52) {
-          x = (b5 >> (f - 2 * kCombos) & 1) ? 1.f : 0.f;
-        } else if (f < 2 * kCombos + 65) {
-          x = (ranks >> (f - 2 * kCombos - 52) & 1) ? 1.f : 0.f;
-        } else {
-          x = f == kBoundaryInput - 3 ? fpot : f == kBoundaryInput - 2 ? fstack : fpl;
-        }
-        v[e] = x;
-      }
-      if (BF16) {
-        __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
-        uint2 w;
-        w.x = *reinterpret_cast<unsigned*>(&a);
-        w.y = *reinterpret_cast<unsigned*>(&b);
-        reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(out) + row)[q] = w;
+    for (int e = 0; e < E; ++e) {
+      const int f = E * q + e;
+      float y;
+      if (f < 2 * kCombos) {
+        int a, b;
+        combo_cards(f - kCombos, a, b);
+        y = a == river || b == river ? 0.f : rr[f];
+      } else if (f < 2 * kCombos + 52) {
+        y = (b5 >> (f - 2 * kCombos) & 1) ? 1.f : 0.f;
+      } else if (f < 2 * kCombos + 65) {
+        y = (ranks >> (f - 2 * kCombos - 52) & 1) ? 1.f : 0.f;
       } else {
-        reinterpret_cast<float4*>(static_cast<float*>(out) + row)[q] = make_float4(v[0], v[1], v[2], v[3]);
+        y = f == kBoundaryInput - 3 ? fpot : f == kBoundaryInput - 2 ? fstack : (float)player;
       }
+      x[e] = bits(y);
+    }
+    put(o0 + (size_t)ri * kVec + q, pack(x));  // the second player's rows follow the first's
+  }
+  for (int q = threadIdx.x; q < kPlain; q += blockDim.x) {
+    uint32_t v[E];
+    int c1[E], c2[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int f = E * q + e;
+      v[e] = bits(rr[f]);
+      combo_cards(f < kCombos ? f : f - kCombos, c1[e], c2[e]);
+    }
+#pragma unroll 4
+    for (int ri = 0; ri < kRivers; ++ri) {
+      const int river = s_river[ri];
+      uint32_t x[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) x[e] = c1[e] == river || c2[e] == river ? 0u : v[e];
+      const uint4 w = pack(x);
+      put(o0 + (size_t)ri * kVec + q, w);
+      put(o1 + (size_t)ri * kVec + q, w);
     }
   }
 }
 
-cudaError_t launch_boundary_encode(int n, const uint8_t* boards, const float* pots, const float* stacks,
-                                   const float* reach, void* out, int bf16, cudaStream_t s) {
+cudaError_t launch_boundary_encode(int n, const ItemMeta& meta, const float* reach, void* out, int bf16,
+                                   cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   if (bf16)
-    k_boundary_encode<true><<<2 * n, 256, 0, s>>>(boards, pots, stacks, reach, out);
+    k_boundary_encode<true><<<n, kEncodeThreads, 0, s>>>(meta, reach, out, ((uintptr_t)out & 15) == 0);
   else
-    k_boundary_encode<false><<<2 * n, 256, 0, s>>>(boards, pots, stacks, reach, out);
+    k_boundary_encode<false><<<n, kEncodeThreads, 0, s>>>(meta, reach, out, true);
   return cudaGetLastError();
 }
 
@@ -315,16 +447,23 @@ cudaError_t launch_pack_records(const SpotDev* spots, int n, const float* ranges
   return cudaGetLastError();
 }
 
-cudaError_t launch_boundary_river_reduce(int n, const uint8_t* boards, const float* denorm, const void* net,
-                                         int net_bf16, const float* reach, const int32_t* hands, int H, float* out,
+cudaError_t launch_boundary_river_reduce(int n, const ItemMeta& meta, const void* net, int net_bf16,
+                                         const float* reach, const int32_t* hands, int H, float* out,
                                          cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   if (net_bf16)
-    k_boundary_river_reduce<__nv_bfloat16><<<2 * n, 256, 0, s>>>(
-        n, boards, denorm, static_cast<const __nv_bfloat16*>(net), reach, hands, H, out);
+    k_boundary_river_reduce<__nv_bfloat16><<<2 * n, kReduceThreads, 0, s>>>(meta, static_cast<const __nv_bfloat16*>(net), reach,
+                                                                 hands, H, out, ((uintptr_t)net & 3) == 0);
   else
-    k_boundary_river_reduce<float><<<2 * n, 256, 0, s>>>(n, boards, denorm, static_cast<const float*>(net), reach,
-                                                         hands, H, out);
+    k_boundary_river_reduce<float><<<2 * n, kReduceThreads, 0, s>>>(meta, static_cast<const float*>(net), reach, hands, H, out,
+                                                         ((uintptr_t)net & 7) == 0);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_river_average_grad(int n, const ItemMeta& meta, const float* reach, const float* g, float* gy,
+                                      cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  k_river_average_grad<<<2 * n, kReduceThreads, 0, s>>>(meta, reach, g, gy, ((uintptr_t)gy & 7) == 0);
   return cudaGetLastError();
 }
 

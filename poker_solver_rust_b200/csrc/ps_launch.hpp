@@ -65,13 +65,24 @@ struct GridJob {
   int cluster = 0;                   // set by launch_grid: the CTAs form one cluster (hardware barrier)
 };
 int grid_ctas(int block, const SmemPlan& plan);
+// Host-side metadata of up to kMetaItems boundary items, passed to the datagen
+// kernels by value: their 4-card boards and two numbers per item.  12 KB of
+// kernel parameters replace three copies through a staging buffer.
+constexpr int kMetaItems = 1024;
+struct ItemMeta {
+  uint8_t board[kMetaItems][4];
+  float a[kMetaItems], b[kMetaItems];
+};
 // Reach-weighted 48-river average of boundary-network outputs (ps_datagen.cu):
-// boards [n][4], denorm [n] (pot + stack), net [n][2][48][1326] (f32, or bf16
-// when net_bf16), reach [n][2][1326], hands [H] combo indices, out [n][2][H];
-// all device pointers.
-cudaError_t launch_boundary_river_reduce(int n, const uint8_t* boards, const float* denorm, const void* net,
-                                         int net_bf16, const float* reach, const int32_t* hands, int H, float* out,
+// n <= kMetaItems items with meta.a = pot + stack, net [n][2][48][1326] (f32,
+// or bf16 when net_bf16), reach [n][2][1326], hands [H] combo indices, out
+// [n][2][H]; device pointers.  launch_river_average_grad: its gradient with
+// respect to net for g [n][2][1326] (every combo in order), gy like net (f32).
+cudaError_t launch_boundary_river_reduce(int n, const ItemMeta& meta, const void* net, int net_bf16,
+                                         const float* reach, const int32_t* hands, int H, float* out,
                                          cudaStream_t s);
+cudaError_t launch_river_average_grad(int n, const ItemMeta& meta, const float* reach, const float* g, float* gy,
+                                      cudaStream_t s);
 // First layer of a boundary network over every input row of
 // launch_boundary_encode without the rows: base [n][h] (weights times the
 // reach rows), percard [n][52][h] (weights times the reach of the combos
@@ -100,11 +111,12 @@ cudaError_t launch_spot_combo(const SpotDev* spots, int n, int which, const floa
 // every item, player and river card not on the item's board: [n][2][48][2720],
 // oop reach | ip reach (1326 each, zeroed where a hand holds the river card) |
 // 52 board one-hot | 13 rank presence | pot/(pot+stack) | stack/(pot+stack) | player.
-// boards [n][4], pots [n], stacks [n], reach [n][2][1326]; device pointers;
-// out is f32, or bf16 (round to nearest even) when bf16 != 0.
+// n <= kMetaItems items with meta.a = pot and meta.b = stack; reach
+// [n][2][1326] and out are device pointers; out is f32, or bf16 (round to
+// nearest even) when bf16 != 0.
 constexpr int kBoundaryInput = 2720;
-cudaError_t launch_boundary_encode(int n, const uint8_t* boards, const float* pots, const float* stacks,
-                                   const float* reach, void* out, int bf16, cudaStream_t s);
+cudaError_t launch_boundary_encode(int n, const ItemMeta& meta, const float* reach, void* out, int bf16,
+                                   cudaStream_t s);
 // Per-spot fields of a training record that the device descriptor lacks.
 struct RecordMeta {
   float pot, stack;   // starting pot and effective stack

@@ -19,9 +19,12 @@ respect to the network's parameters:
 
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import torch
 
+from . import _native as N
 from .datagen import boundary_encode, boundary_river_reduce, solve_with_boundary_net
 
 _PAIRS = None
@@ -46,25 +49,45 @@ def river_keep_mask(boards, device):
     return (pr[None, None, :, 0] != rivers[:, :, None]) & (pr[None, None, :, 1] != rivers[:, :, None])
 
 
+def _river_average_grad(boards, scale, reach, g):
+    """[n, 2, 48, 1326] gradient with respect to the network outputs (f32 CUDA tensors)."""
+    b = np.ascontiguousarray(boards, np.uint8).reshape(-1, 4)
+    n = len(b)
+    reach, g = reach.contiguous(), g.contiguous()
+    gy = torch.empty((n, 2, 48, 1326), dtype=torch.float32, device=g.device)
+    N.check(N.lib().ps_river_average_grad(
+        n, b.ctypes.data_as(C.POINTER(C.c_uint8)), scale.ctypes.data_as(C.POINTER(C.c_float)),
+        C.c_void_p(reach.data_ptr()), C.c_void_p(g.data_ptr()), C.c_void_p(gy.data_ptr()),
+        C.c_void_p(torch.cuda.current_stream(g.device).cuda_stream)))
+    return gy
+
+
 class RiverAverage(torch.autograd.Function):
     """The reach-weighted 48-river average (ps_boundary_river_reduce, combo
     layout) as a function of the network outputs y [n, 2, 48, 1326]; reach
     and the scale are constants.  Backward: dB/dy[i,p,r,c] = scale_i *
     W[i,p,r] * keep[i,r,c] / sum_r' W[i,p,r'] keep[i,r',c], where W[i,p,r] is
-    the opponent's reach on combos free of river r (gpu_boundary_eval.rs:146-161)."""
+    the opponent's reach on combos free of river r (gpu_boundary_eval.rs:146-161),
+    in f64: one kernel (ps_river_average_grad) for a plain f32 gradient, the
+    same formula in torch where the gradient itself is differentiated."""
 
     @staticmethod
     def forward(ctx, y, boards, scale, reach):
         combos = torch.arange(1326, dtype=torch.int32, device=y.device)
         scale = np.asarray(scale, np.float32)
         out = boundary_river_reduce(boards, scale, np.zeros(len(scale), np.float32), y.detach(), reach, combos)
-        ctx.save_for_backward(reach, torch.as_tensor(scale, device=y.device))
+        ctx.save_for_backward(reach)
         ctx.boards = boards
+        ctx.scale = scale.copy()
         return out
 
     @staticmethod
     def backward(ctx, g):
-        reach, s = ctx.saved_tensors
+        (reach,) = ctx.saved_tensors
+        if (type(g) is torch.Tensor and g.is_cuda and g.dtype == reach.dtype == torch.float32
+                and not (torch.is_grad_enabled() and g.requires_grad)):
+            return _river_average_grad(ctx.boards, ctx.scale, reach, g), None, None, None
+        s = torch.as_tensor(ctx.scale, device=g.device)
         keep = river_keep_mask(ctx.boards, g.device).to(torch.float64)  # [n, 48, 1326]
         opp = reach.flip(1).to(torch.float64)  # player 0 weighted by IP reach, player 1 by OOP reach
         W = torch.einsum("npc,nrc->npr", opp, keep)  # [n, 2, 48]
