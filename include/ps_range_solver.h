@@ -255,15 +255,18 @@ typedef struct ps_batch_opts {
                              autotuner then also tries all of them) */
   int32_t instances_per_cta; /* spots of one tree shape a CTA solves in lockstep, 1..4
                                 (0 = 1); they share each step's barrier */
-  int32_t scheduler;      /* PS_SCHED_DEFAULT (0): dataflow for batches of more spots than SMs,
-                             step-synchronous otherwise; PS_SCHED_STEP (1): every CTA walks
+  int32_t scheduler;      /* PS_SCHED_DEFAULT (0): dataflow for batches of 16 spots or more
+                             (of more spots than SMs when block_threads, ctas_per_sm,
+                             instances_per_cta or stage_tables is set), step-synchronous
+                             otherwise; PS_SCHED_STEP (1): every CTA walks
                              its spot's steps with one barrier per step (k_solve);
                              PS_SCHED_FLOW (2): each CTA holds several spots at once and its
                              warps take the ready items of any of them (k_flow).  Results
                              are the same bits either way. */
   int32_t flow_threads;   /* dataflow: threads per CTA, a multiple of 32 from 128 to 1024
                              (0 = 1024; with block_threads = -1 the autotuner chooses) */
-  int32_t flow_spots_per_cta; /* dataflow: spots a CTA holds at once, 1..8 (0 = 3, or autotuned) */
+  int32_t flow_spots_per_cta; /* dataflow: spots a CTA holds at once, 1..8 (0 = as many as the
+                                 batch has per SM, at most 3, or autotuned) */
   int32_t node_parts;     /* dataflow: column blocks each node op is cut into, 1..16
                              (0 = 3, or autotuned) */
 } ps_batch_opts;

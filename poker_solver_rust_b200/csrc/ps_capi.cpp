@@ -63,6 +63,7 @@ constexpr int kMaxInstances = 4;  // spots per CTA in lockstep (ps_batch_opts.in
 // single games with at most this many acting hand-edges (sum over decision
 // edges of the actor's hands) run on one thread-block cluster (Batch::build)
 constexpr int64_t kClusterMaxEdgeHands = 131072;
+constexpr int kFlowMinSpots = 16;  // batches from this size on run the dataflow kernel by default
 std::mutex g_dev_mu;
 std::mutex g_tune_mu;
 
@@ -672,11 +673,22 @@ struct Batch {
     {
       const int sched = opts ? opts->scheduler : PS_SCHED_DEFAULT;
       if (sched < PS_SCHED_DEFAULT || sched > PS_SCHED_FLOW) return fail(PS_ERR_INVALID, "unknown scheduler");
-      flow = sched == PS_SCHED_FLOW || (sched == PS_SCHED_DEFAULT && n > dc->nsm);
+      // the dataflow kernel is the faster one also where every spot has an SM
+      // to itself (16 river spots 54 against 121 ms, 100: 69 against 155, 148:
+      // 66 against 153); a handful of spots, and a caller that shapes or tunes
+      // the step-synchronous CTAs of so few, keep that schedule
+      const bool shaped = opts && (opts->block_threads != 0 || opts->ctas_per_sm > 0 || opts->instances_per_cta > 0 ||
+                                   opts->stage_tables >= 0);
+      flow = sched == PS_SCHED_FLOW ||
+             (sched == PS_SCHED_DEFAULT && (n > dc->nsm || (n >= kFlowMinSpots && !shaped)));
       if (flow) {
         int fb = opts && opts->flow_threads > 0 ? opts->flow_threads : 1024;
         fb = std::max(128, std::min(kMaxFlowThreads, (fb / 32) * 32));
-        const int fl = opts && opts->flow_spots_per_cta > 0 ? opts->flow_spots_per_cta : 3;
+        // spots per CTA: as many as the batch has for each SM, at most 3 (the
+        // next would overflow L2: 4096 river spots 413 ms with 3, 594 with 4;
+        // 301 spots 67-68 ms with 1, 2 or 3, 1500 spots 273, 183, 154)
+        const int fl = opts && opts->flow_spots_per_cta > 0 ? opts->flow_spots_per_cta
+                                                            : std::min(3, (n + dc->nsm - 1) / dc->nsm);
         const int fp = opts && opts->node_parts > 0 ? opts->node_parts : 3;
         if (fl > kMaxFlowLanes || fp > 16) return fail(PS_ERR_INVALID, "flow_spots_per_cta 1..8, node_parts 1..16");
         const int rc = adopt_flow(fb, opts && opts->scan_buffers > 0 ? opts->scan_buffers : fb / 64, fl, fp,
@@ -810,7 +822,7 @@ struct Batch {
     occ = flow_occupancy(b, pl);
     if (occ < 1 || lanes > pl.warps) return false;
     if (cap_ctas > 0) occ = std::min(occ, cap_ctas);
-    g = std::max(1, std::min((nspots + lanes - 1) / lanes, dc->nsm * occ));
+    g = std::max(1, std::min(nspots, dc->nsm * occ));
     return true;
   }
 
@@ -939,7 +951,7 @@ struct Batch {
         if (e == cudaSuccess) e = cudaEventRecord(ev[2], stream);
         if (e == cudaSuccess)
           e = launch_flow(d_sample, nq, q, d_cnt, d_disc, jb, d_tz, d_tscratch, scratch_floats, d_te, d_ti, d_err,
-                          g, c.b, c.lanes, c.parts, pl, stream);
+                          g, c.b, c.lanes, c.parts, pl, stream, !items.empty());
         if (e == cudaSuccess) e = cudaEventRecord(ev[3], stream);
       }
       if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
@@ -1044,7 +1056,7 @@ struct Batch {
       CU(cudaMemsetAsync(d_cnt, 0, sizeof(int), stream));
       CU(cudaEventRecord(ev[2], stream));
       CU(launch_flow(d_sample, ns, d_ids, d_cnt, d_disc, job, d_tg, d_tscratch, scratch_floats, d_te, d_ti, d_err, g,
-                     c[0], c[2], c[3], pl, stream));
+                     c[0], c[2], c[3], pl, stream, !items.empty()));
       CU(cudaEventRecord(ev[3], stream));
       CU(cudaStreamSynchronize(stream));
       float ms = 0;
@@ -1083,7 +1095,7 @@ struct Batch {
     if (flow)
       return launch_flow(d_spots, (int)games.size(), d_order, d_counter, d_disc, job, d_target, d_scratch,
                          scratch_floats, d_expl, d_iters, d_err, flow_grid, flow_block, flow_lanes, flow_parts,
-                         flow_plan, stream);
+                         flow_plan, stream, !items.empty());
     return launch_solve(d_spots, ninst, inst_k, d_inst, d_counter, d_disc, job, d_target, d_scratch, scratch_floats,
                         d_expl, d_iters, d_err, grid, block, plan, stream);
   }
@@ -1401,8 +1413,7 @@ struct Batch {
       CU(cudaMemsetAsync(d_counter, 0, sizeof(int), stream));
       SolveJob job{0, 0, 0, 0};
       job.adjoint = 1;
-      CU(launch_solve(d_spots, ninst, inst_k, d_inst, d_counter, d_disc, job, d_target, d_scratch, scratch_floats,
-                      d_expl, d_iters, d_err, grid, block, plan, stream));
+      CU(launch_job(job));
     }
     CU(cudaStreamSynchronize(stream));
     return check_err();

@@ -568,7 +568,7 @@ __device__ __forceinline__ void lookup_sweep(const Rec* rec, float* dst, int h0,
   }
 }
 
-template <bool GEN, bool SPLIT = false, bool CTA = false>
+template <bool GEN, bool SPLIT = false, bool CTA = false, bool BOUNDARY = true>
 __device__ __forceinline__ void warp_terms_inl(const Ctx& c, const Op* ops, int n, int p) {
   static_assert(!CTA || (SPLIT && !GEN), "CTA runs are solve-pass runs of lone spots");
   PHASE_T0(t_scan);
@@ -718,7 +718,7 @@ __device__ __forceinline__ void warp_terms_inl(const Ctx& c, const Op* ops, int 
                         }));
         return keep_if(f.y & FOLD_VALID, v);
       });
-    } else {  // depth boundary (evaluation.rs:544-605)
+    } else if (BOUNDARY) {  // depth boundary (evaluation.rs:544-605)
       const float scale = nd.payoff_scale;
       const float* brow = sp.bcfv + ((size_t)nd.boundary * 2 + p) * c.vstride;
       float* grow = GEN && c.bgrad ? c.bgrad + ((size_t)nd.boundary * 2 + p) * c.vstride : nullptr;
@@ -1320,7 +1320,10 @@ __global__ void PS_SOLVE_BOUNDS k_solve(const SpotDev* __restrict__ spots, int n
 // its claim.
 constexpr int kMaxLanes = 8;
 constexpr int kMaxFlowBlock = 1024;
-enum LanePhase : int { LP_BR0 = 0, LP_BR1, LP_AVG0, LP_AVG1, LP_DCFR0, LP_DCFR1, LP_EPI0, LP_EPI1, LP_RETIRED };
+// (even phases are passes of traverser 0; LP_ADJ0 / 1 are the forward passes of
+// an adjoint job, LP_ADJ2 / 3 its transposed passes)
+enum LanePhase : int { LP_BR0 = 0, LP_BR1, LP_AVG0, LP_AVG1, LP_DCFR0, LP_DCFR1, LP_EPI0, LP_EPI1,
+                       LP_ADJ0, LP_ADJ1, LP_ADJ2, LP_ADJ3, LP_RETIRED };
 
 struct Lane {
   unsigned long long wt, wn;  // claims of terminal runs / node-op parts: count << 20 | next
@@ -1348,6 +1351,14 @@ __device__ __forceinline__ int try_claim(unsigned long long* w) {
   const unsigned nxt = (unsigned)(old & 0xFFFFFull), cnt = (unsigned)((old >> 20) & 0xFFFFFull);
   return nxt < cnt ? (int)nxt : -1;
 }
+
+// Instantiations of k_flow by what its terminal items can meet: batches
+// without depth boundaries, batches with them (boundary values, the epilogue's
+// boundary reach) and the adjoint.  Each holds only the code it runs, which
+// its registers and instruction fetches are tight on: with the adjoint's
+// branches in the one kernel 4096 river spots took 454 ms, against 413 in the
+// first instantiation.
+enum FlowJob { FLOW_PLAIN = 0, FLOW_BOUNDARY = 1, FLOW_ADJOINT = 2 };
 
 struct FlowArgs {
   const SpotDev* spots;
@@ -1437,10 +1448,12 @@ __device__ int lane_after_iterations(const Lane& L, const FlowArgs& A) {
 
 // Binds the lane to the next spot of the queue (lane 0 of the calling warp);
 // false when the queue is empty and the lane retires.  The lane starts before
-// the first step of its first pass (step -1).
-__device__ bool lane_bind(Lane& L, const FlowArgs& A, float* my_scratch, const SmemPlan& plan) {
+// the first step of its first pass (step -1).  first >= 0: the queue place a
+// lane starts with; the places after every lane's first come from the counter.
+__device__ bool lane_bind(Lane& L, const FlowArgs& A, float* my_scratch, const SmemPlan& plan, int first = -1) {
   for (;;) {
-    const int q = atomicAdd(A.counter, 1);
+    const int q = first >= 0 ? first : atomicAdd(A.counter, 1) + (int)gridDim.x * A.lanes;
+    first = -1;
     if (q >= A.ninst) {
       L.phase = LP_RETIRED;
       return false;
@@ -1454,7 +1467,10 @@ __device__ bool lane_bind(Lane& L, const FlowArgs& A, float* my_scratch, const S
     }
     const SolveJob& j = A.job;
     int phase;
-    if (j.checks) {
+    if (j.adjoint) {
+      L.t = 0;
+      phase = LP_ADJ0;
+    } else if (j.checks) {
       L.t = 0;
       phase = LP_BR0;  // the exploitability before the first iteration
     } else {
@@ -1519,6 +1535,10 @@ __device__ int lane_pass_end(Lane& L, const FlowArgs& A) {
       if (next < 0) L.iters = L.t;
     }
     next = __shfl_sync(0xffffffffu, next, 0);
+  } else if (L.phase >= LP_ADJ0) {  // root values, then the gradients of the weights
+    float* dst = L.phase <= LP_ADJ1 ? sp.root_out[p] : sp.adj_dw[p];
+    for (int h = lane; h < sp.H[p]; h += 32) dst[h] = root[h];
+    return L.phase < LP_ADJ3 ? L.phase + 1 : -1;
   } else {  // LP_EPI0 / LP_EPI1: root values under the average strategy
     if (sp.root_out[p])
       for (int h = lane; h < sp.hs[p]; h += 32) sp.root_out[p][h] = root[h];
@@ -1577,14 +1597,15 @@ __device__ bool lane_move(Lane& L, const FlowArgs& A, const SmemPlan& plan) {
 
 // Runs item `idx` of the lane's current step: a terminal run (term) or a
 // node-op column block.
-__device__ void lane_item(const Lane& L, const FlowArgs& A, int term, int idx, float* buf, int bufs) {
+template <int JOB>
+__device__ __forceinline__ void lane_item(const Lane& L, const FlowArgs& A, int term, int idx, float* buf, int bufs) {
   const SpotDev& sp = A.spots[L.spot];
-  const int p = lane_player(L.phase), o = p ^ 1, mode = lane_mode(L.phase);
+  const int p = lane_player(L.phase), o = p ^ 1, mode = JOB == FLOW_ADJOINT ? M_AVG : lane_mode(L.phase);
   Ctx c;
   c.sp = &sp;
   c.slots = L.slots;
   c.vstride = sp.vstride;
-  c.root_reach = sp.w[o];
+  c.root_reach = JOB == FLOW_ADJOINT && L.phase >= LP_ADJ2 ? sp.adj_g[o] : sp.w[o];
   c.grid = 0;
   c.bar = nullptr;
   c.gred = nullptr;
@@ -1592,10 +1613,10 @@ __device__ void lane_item(const Lane& L, const FlowArgs& A, int term, int idx, f
   c.err = A.err;
   c.buf = buf;
   c.bufs = bufs;
-  c.owner = -1;
+  c.owner = JOB == FLOW_ADJOINT && L.phase >= LP_ADJ2 ? o : -1;
   c.signed_reach = 0;
-  c.bgrad = nullptr;
-  c.breach = L.phase >= LP_EPI0 ? sp.breach : nullptr;
+  c.bgrad = JOB == FLOW_ADJOINT ? sp.bgrad : nullptr;
+  c.breach = JOB == FLOW_BOUNDARY && L.phase >= LP_EPI0 ? sp.breach : nullptr;
   c.red = nullptr;
   c.split = 0;
   c.part = 0;
@@ -1610,10 +1631,10 @@ __device__ void lane_item(const Lane& L, const FlowArgs& A, int term, int idx, f
   const Discount dc = mode == M_DCFR ? A.disc[L.t] : Discount{0.f, 0.f, 0.f, 0.f};
   if (term) {
     const Op* lead = sp.ops[p] + L.begin + L.n_elem + sp.groups[p][L.gbegin + idx];
-    if (c.breach)
+    if (JOB != FLOW_PLAIN && L.phase >= LP_EPI0)
       warp_terms_inl<true>(c, lead, lead->na, p);
-    else
-      warp_terms_inl<false>(c, lead, lead->na, p);
+    else if (JOB != FLOW_ADJOINT)
+      warp_terms_inl<false, false, false, JOB == FLOW_BOUNDARY>(c, lead, lead->na, p);
     return;
   }
   const int P = L.parts;
@@ -1650,6 +1671,7 @@ constexpr long long kFlowIdleNs = 2000000000LL;  // 2 s without any finished ste
 #endif
 constexpr unsigned kFlowSleepMinNs = PS_FLOW_SLEEP_MIN, kFlowSleepMaxNs = PS_FLOW_SLEEP_MAX;  // idle back-off
 
+template <int JOB>
 __global__ void __launch_bounds__(kMaxFlowBlock, 1) k_flow(FlowArgs A, SmemPlan plan) {
   extern __shared__ float4 smem4[];
   char* smem = reinterpret_cast<char*>(smem4);
@@ -1674,7 +1696,12 @@ __global__ void __launch_bounds__(kMaxFlowBlock, 1) k_flow(FlowArgs A, SmemPlan 
     if (lane == 0) {
       L.wt = L.wn = 0ull;
       L.done = L.total = 0;
-      bound = lane_bind(L, A, A.scratch + ((size_t)blockIdx.x * K + warp) * A.scratch_floats, plan);
+      // lane by lane over the CTAs, back and forth: the queue is in falling
+      // cost, so every CTA starts with spots of about the same total (bound
+      // as the warps came, the first CTAs took the costliest spots each)
+      const int b = warp & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+      bound = lane_bind(L, A, A.scratch + ((size_t)blockIdx.x * K + warp) * A.scratch_floats, plan,
+                        warp * (int)gridDim.x + b);
       if (!bound) atomicAdd(&s_retired, 1);
     }
     if (__shfl_sync(0xffffffffu, bound, 0) && lane_move(L, A, plan) && lane == 0) atomicAdd(&s_retired, 1);
@@ -1710,7 +1737,7 @@ __global__ void __launch_bounds__(kMaxFlowBlock, 1) k_flow(FlowArgs A, SmemPlan 
       term = __shfl_sync(0xffffffffu, term, 0);
       __syncwarp();
       Lane& L = lanes[k];
-      lane_item(L, A, term, idx, buf, plan.bufs);
+      lane_item<JOB>(L, A, term, idx, buf, plan.bufs);
       __threadfence_block();  // every lane's writes of the item before its count
       __syncwarp();
       int last = 0;
@@ -2188,29 +2215,41 @@ cudaError_t launch_solve(const SpotDev* spots, int ninst, int K, const int* inst
   return cudaGetLastError();
 }
 
+static const void* flow_kernel(int kind) {
+  return kind == FLOW_ADJOINT    ? (const void*)k_flow<FLOW_ADJOINT>
+         : kind == FLOW_BOUNDARY ? (const void*)k_flow<FLOW_BOUNDARY>
+                                 : (const void*)k_flow<FLOW_PLAIN>;
+}
+
 cudaError_t launch_flow(const SpotDev* spots, int ninst, const int* inst, int* counter, const Discount* disc,
                         const SolveJob& job, const float* target, float* scratch, size_t scratch_floats,
                         float* out_expl, int* out_iters, int* err, int grid, int block, int lanes, int node_parts,
-                        const SmemPlan& plan, cudaStream_t s) {
+                        const SmemPlan& plan, cudaStream_t s, bool boundaries) {
   if (block < 64 || block > kMaxFlowBlock || block % 32 || lanes < 1 || lanes > kMaxLanes || lanes > block / 32 ||
-      node_parts < 1 || node_parts > 16 || plan.bufs < 1 || plan.bufs > block / 32 || job.adjoint || job.t0 < 0 ||
-      job.t1 < job.t0 || (job.checks && job.t0 != 0))
+      node_parts < 1 || node_parts > 16 || plan.bufs < 1 || plan.bufs > block / 32 || job.t0 < 0 ||
+      job.t1 < job.t0 || (job.checks && job.t0 != 0) || (job.adjoint && (job.checks || job.t1 != job.t0)))
     return cudaErrorInvalidValue;
   size_t smem = plan.total();
-  cudaError_t e = set_smem((const void*)k_flow, smem);
+  const int kind = job.adjoint ? FLOW_ADJOINT : boundaries ? FLOW_BOUNDARY : FLOW_PLAIN;
+  cudaError_t e = set_smem(flow_kernel(kind), smem);
   if (e != cudaSuccess) return e;
   FlowArgs A{spots, ninst, inst, counter, disc, job, target, scratch, scratch_floats, out_expl, out_iters, err,
              lanes, node_parts};
-  k_flow<<<grid, block, smem, s>>>(A, plan);
-  return cudaGetLastError();
+  SmemPlan pl = plan;
+  void* args[] = {(void*)&A, (void*)&pl};
+  return cudaLaunchKernel(flow_kernel(kind), dim3(grid), dim3(block), args, smem, s);
 }
 
 int flow_occupancy(int block, const SmemPlan& plan) {
-  int n = 0;
   size_t smem = plan.total();
-  if (set_smem((const void*)k_flow, smem) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_flow, block, smem) != cudaSuccess) return 0;
-  return n;
+  int least = 1 << 30;  // the launch shape serves every job of the batch
+  for (int kind : {FLOW_PLAIN, FLOW_BOUNDARY, FLOW_ADJOINT}) {
+    int n = 0;
+    if (set_smem(flow_kernel(kind), smem) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, flow_kernel(kind), block, smem) != cudaSuccess) return 0;
+    least = n < least ? n : least;
+  }
+  return least;
 }
 
 int grid_ctas(int block, const SmemPlan& plan) {

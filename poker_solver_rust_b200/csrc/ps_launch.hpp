@@ -183,7 +183,7 @@ cudaError_t launch_solve(const SpotDev* spots, int ninst, int K, const int* inst
 // Dataflow batched solve (k_flow): each CTA holds `lanes` spots at once, each
 // at its own step; warps claim the steps' items (terminal runs; node ops cut
 // into node_parts column blocks) instead of waiting at per-step barriers.
-// The same jobs as launch_solve except the adjoint; inst: [ninst] spot ids in
+// The same jobs as launch_solve (boundaries: some spot has depth boundaries); inst: [ninst] spot ids in
 // the order they are handed out; scratch holds lanes * scratch_floats floats
 // per CTA.  Results equal launch_solve's bit for bit.
 constexpr int kMaxFlowThreads = 1024;
@@ -191,7 +191,7 @@ constexpr int kMaxFlowLanes = 8;
 cudaError_t launch_flow(const SpotDev* spots, int ninst, const int* inst, int* counter, const Discount* disc,
                         const SolveJob& job, const float* target, float* scratch, size_t scratch_floats,
                         float* out_expl, int* out_iters, int* err, int grid, int block, int lanes, int node_parts,
-                        const SmemPlan& plan, cudaStream_t s);
+                        const SmemPlan& plan, cudaStream_t s, bool boundaries);
 int flow_occupancy(int block, const SmemPlan& plan);  // CTAs per SM (0 = does not fit)
 cudaError_t launch_iterate(const SpotDev* spots, int nspots, const Discount* disc, int t0, int t1,
                            float* scratch, size_t scratch_floats, int* err, int grid, int block,

@@ -560,7 +560,7 @@ class BatchSolver:
                  stage_tables: int = -1, scan_buffers: int = 0, instances_per_cta: int = 0,
                  scheduler: int = 0, flow_threads: int = 0, flow_spots_per_cta: int = 0, node_parts: int = 0):
         """Options as ps_batch_opts (include/ps_range_solver.h).  scheduler:
-        0 = default (dataflow for batches of more spots than SMs), 1 =
+        0 = default (dataflow for batches of 16 spots or more), 1 =
         step-synchronous (one barrier per step), 2 = dataflow; flow_threads,
         flow_spots_per_cta, node_parts shape the dataflow launch (0 = default,
         or autotuned with block_threads = -1)."""
