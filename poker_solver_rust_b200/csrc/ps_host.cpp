@@ -748,9 +748,19 @@ void Game::compile(int p, bool terminals_first) {
   for (size_t i = 0; i < idx.size(); ++i) idx[i] = (int)i;
   std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return blks[x].birth < blks[y].birth; });
   std::vector<int> busy_until;
+  // Blocks of one birth only take slots away, so a size's search goes on where
+  // its last one of that birth ended: a search from slot 0 for every block was
+  // most of a 12,285-node game's 45 ms construction.
+  int birth = -1;
+  std::vector<int> from;  // per block size
   for (int i : idx) {
     Blk& b = blks[i];
-    int s = 0;
+    if (b.birth != birth) {
+      birth = b.birth;
+      std::fill(from.begin(), from.end(), 0);
+    }
+    if ((int)from.size() <= b.size) from.resize(b.size + 1, 0);
+    int& s = from[b.size];
     for (;; ++s) {
       bool ok = true;
       for (int k = 0; k < b.size && ok; ++k)
