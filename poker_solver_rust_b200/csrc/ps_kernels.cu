@@ -400,8 +400,18 @@ __device__ __forceinline__ void op_bwd_opp(const Ctx& c, const Op& op, int p, in
   op_bwd_opp_t<false>(c, op, p, mode);
 }
 
+// finalize only (M_AVG_SAVE): chance cfvalues of the node for four hands, out of line
+__device__ __noinline__ void save_chance_cfv(const SpotDev& sp, const NodeDev& nd, int p, int h, float4 res) {
+  const float v[4] = {res.x, res.y, res.z, res.w};
+  for (int k = 0; k < 4; ++k)
+    if (h + k < sp.H[p]) sp.chcfv[nd.ch_off + h + k] = v[k];
+}
+
 // Chance node: cfv = sum over dealt cards, plus the suit-swapped rows of the
-// isomorphic cards that were not dealt (solver.rs:291-325).
+// isomorphic cards that were not dealt (solver.rs:291-325).  Four hands per
+// lane, eight children's rows in flight: one hand and one dependent row at a
+// time, the warps with a chance node (48 children) held up every other one of
+// a turn game's two widest steps (60 iterations with construction 107 -> 93 ms).
 template <bool SPLIT>
 __device__ __forceinline__ void op_bwd_chance_t(const Ctx& c, const Op& op, int p, int mode) {
   // SPLIT: this item is column block c.part of c.parts (interleaved 32-column blocks)
@@ -416,16 +426,19 @@ __device__ __forceinline__ void op_bwd_chance_t(const Ctx& c, const Op& op, int 
     i0 = sp.iso_off[op.board];
     i1 = sp.iso_off[op.board + 1];
   }
-  for (int h = part * 32 + (threadIdx.x & 31); h < hsp; h += 32 * parts) {
-    float res = cb[h];
-    for (int a = 1; a < na; ++a) res = __fadd_rn(res, cb[(size_t)a * c.vstride + h]);
+  for (int q = part * 32 + (threadIdx.x & 31); q < hsp >> 2; q += 32 * parts) {
+    const int h = q << 2;
+    float4 res = ld4(cb + h);
+#pragma unroll 8
+    for (int a = 1; a < na; ++a) res = add4(res, ld4(cb + (size_t)a * c.vstride + h));
     for (int i = i0; i < i1; ++i) {
       const int ref = sp.iso_ent[2 * i], perm = sp.iso_ent[2 * i + 1];
-      const int hh = sp.iso_perm[p][(size_t)perm * hsp + h];
-      res = __fadd_rn(res, cb[(size_t)ref * c.vstride + hh]);
+      const ushort4 hh = *reinterpret_cast<const ushort4*>(sp.iso_perm[p] + (size_t)perm * hsp + h);
+      const float* row = cb + (size_t)ref * c.vstride;
+      res = add4(res, make_float4(row[hh.x], row[hh.y], row[hh.z], row[hh.w]));
     }
-    dst[h] = res;
-    if (mode == M_AVG_SAVE && nd.ch_player == p && h < sp.H[p]) sp.chcfv[nd.ch_off + h] = res;
+    st4(dst + h, res);
+    if (mode == M_AVG_SAVE && nd.ch_player == p) save_chance_cfv(sp, nd, p, h, res);
   }
 }
 __device__ __forceinline__ void op_bwd_chance(const Ctx& c, const Op& op, int p, int mode) {
