@@ -2544,9 +2544,9 @@ int ps_expected_values(ps_game* G, int player, int detail, float* out) {  // que
     CU(cudaStreamSynchronize(B.stream));
     if ((rc = B.check_err())) return rc;
   } else if (n.chance() && n.ch_off != 0xFFFFFFFFu && ((n.player & PL_MASK) ^ 1) == player) {
-    ret.assign(G->hCH.begin() + n.ch_off, G->hCH.begin() + n.ch_off + H);
+    ret.assign(&G->hCH[n.ch_off], &G->hCH[n.ch_off] + H);
   } else if (!n.chance() && n.ip_off != 0xFFFFFFFFu && player == 1) {
-    ret.assign(G->hIP.begin() + n.ip_off, G->hIP.begin() + n.ip_off + H);
+    ret.assign(&G->hIP[n.ip_off], &G->hIP[n.ip_off] + H);
   } else if (!n.chance() && player == n.player) {
     have_actions = true;
     ret.resize((size_t)n.nch * H);

@@ -41,7 +41,8 @@ static_assert(sizeof(Op) == 16, "Op must stay 16 bytes");
 // holds the run length).  All of a step's ops are independent.
 struct Step {
   int32_t begin;
-  int16_t n_elem, n_term, n_groups, pad;
+  int16_t n_elem, n_term, n_groups;
+  int16_t n_chance;  // the first n_chance node ops are backward chance ops (many children each)
   int32_t gbegin;
 };
 

@@ -864,10 +864,13 @@ void Game::compile(int p, bool terminals_first) {
     push_step(begin, 0, (int)P.ops.size() - begin);
   }
   for (int d = D; d >= 0; --d) {
-    int begin = (int)P.ops.size();
-    for (size_t n : at[d]) {
+    int begin = (int)P.ops.size(), n_chance = 0;
+    std::vector<size_t> nodes = at[d];  // chance ops first: a step's widest ops are split finest
+    std::stable_partition(nodes.begin(), nodes.end(), [&](size_t n) { return arena[n].chance(); });
+    for (size_t n : nodes) {
       const ArenaNode& a = arena[n];
       if (a.terminal()) continue;
+      n_chance += a.chance();
       Op o{};
       o.node = (uint32_t)n;
       o.na = (uint8_t)a.nch;
@@ -889,7 +892,9 @@ void Game::compile(int p, bool terminals_first) {
         if (arena[n].terminal()) terms.push_back(n);
       emit_terminals(terms);
     }
+    const size_t before = P.steps.size();
     push_step(begin, ne, (int)P.ops.size() - begin - ne);
+    if (P.steps.size() > before) P.steps.back().n_chance = (int16_t)n_chance;
   }
   // Verification: replay the pass step by step with the meaning of every
   // slot.  Each read must find the vector the op expects; within a step no

@@ -957,20 +957,48 @@ __device__ __noinline__ void run_pass_split(const Ctx& c, int p, const Discount 
     }
     const int busy = cta_runs ? ng * nw0 : min(ng * TP, nb);
     // node ops in up to 16 parts: a 1128-hand row is 282 float4 columns, so 9
-    // parts cover it in one round
-    const int P = ne > 0 ? max(1, min(16, (nw - busy) / ne)) : 1;
-    const int start = busy % nw;
+    // parts (cols) cover it in one round.  A step of more ops than warps takes
+    // the parts that waste least of its last round, and chance ops (48 children
+    // each) always go a round of columns to a warp: 60 iterations of the turn
+    // game with its construction 93 -> 76 ms.
+    const int cols = (sp.hs[p] + 127) >> 7;
+    // (a thin step, the usual one of a small tree, meets no integer division:
+    // each is about 100 cycles of the step's 5,000)
+    int P = 1;
+    if (ne > 0) P = 16 * ne <= nw - busy ? 16 : max(1, (nw - busy) / ne);
+    if (P == 1 && ne > 1) {
+      int best = ((ne + nw - 1) / nw) * cols;
+      for (int k = 2; k <= min(cols, 9); ++k) {
+        const int cost = ((ne * k + nw - 1) / nw) * ((cols + k - 1) / k);
+        if (cost < best) {
+          best = cost;
+          P = k;
+        }
+      }
+    }
+    int w0 = gw - (busy < nw ? busy : 0);  // this warp's first item (busy <= nw)
+    if (w0 < 0) w0 += nw;
     Ctx cw = c;
+    const int nc = st.n_chance;
+    if (nc > 0) {
+      cw.parts = min(cols, 16);
+      const int items = nc * cw.parts;
+      for (int i = w0; i < items; i += nw) {
+        cw.part = i % cw.parts;
+        op_bwd_chance_t<true>(cw, sp.ops[p][st.begin + i / cw.parts], p, mode);
+      }
+      w0 = (w0 + nw - items % nw) % nw;  // the other ops go on behind them
+    }
     cw.parts = P;
-    for (int i = (gw - start + nw) % nw; i < ne * P; i += nw) {
-      const Op op = sp.ops[p][st.begin + i / P];
-      cw.part = i % P;
+    for (int i = w0; i < (ne - nc) * P; i += nw) {
+      const int k = P == 16 ? i >> 4 : i / P;
+      const Op op = sp.ops[p][st.begin + nc + k];
+      cw.part = i - k * P;
       switch (op.type) {
         case OP_FWD_OPP: op_fwd_opp_t<true>(cw, op, o, mode); break;
         case OP_FWD_CHANCE: op_fwd_chance_t<true>(cw, op, o); break;
         case OP_BWD_TRAV: op_bwd_trav_t<true>(cw, op, p, dc, mode); break;
         case OP_BWD_OPP: op_bwd_opp_t<true>(cw, op, p, mode); break;
-        case OP_BWD_CHANCE: op_bwd_chance_t<true>(cw, op, p, mode); break;
         default: break;
       }
     }
