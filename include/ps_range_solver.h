@@ -220,6 +220,11 @@ int ps_river_average_grad(int32_t n, const uint8_t* boards, const float* scale, 
 int ps_boundary_first_layer(int32_t n, const uint8_t* boards, const float* pots, const float* stacks,
                             const float* base, const float* percard, const float* wcols, const float* bias, int32_t h,
                             void* out, int32_t out_bf16, void* stream);
+/* The same without base: it is half the sum of percard over the 52 cards, since
+ * every combo holds two. */
+int ps_boundary_first_layer_cards(int32_t n, const uint8_t* boards, const float* pots, const float* stacks,
+                                  const float* percard, const float* wcols, const float* bias, int32_t h, void* out,
+                                  int32_t out_bf16, void* stream);
 
 /* ---- navigation and queries (game/query.rs) ---- */
 int ps_back_to_root(ps_game* g);

@@ -108,6 +108,7 @@ _sig("ps_boundary_reach", i32, vp, P(f32))
 _sig("ps_boundary_river_reduce", i32, i32, P(C.c_uint8), P(f32), P(f32), vp, i32, vp, vp, i32, vp, vp)
 _sig("ps_river_average_grad", i32, i32, P(C.c_uint8), P(f32), vp, vp, vp, vp)
 _sig("ps_boundary_first_layer", i32, i32, P(C.c_uint8), P(f32), P(f32), vp, vp, vp, vp, i32, vp, i32, vp)
+_sig("ps_boundary_first_layer_cards", i32, i32, P(C.c_uint8), P(f32), P(f32), vp, vp, vp, i32, vp, i32, vp)
 _sig("ps_eval_fixed_strategy_adjoint", i32, vp, P(f32), P(f32), P(f32), P(f32), P(f32), P(f32), P(f32))
 _sig("ps_num_private_hands", i32, vp, i32)
 _sig("ps_private_cards", i32, vp, i32, P(C.c_uint8))

@@ -2045,39 +2045,35 @@ int ps_river_average_grad(int32_t n, const uint8_t* boards, const float* scale, 
       });
 }
 
+static int first_layer(int32_t n, const uint8_t* boards, const float* pots, const float* stacks, const float* base,
+                       const float* percard, const float* wcols, const float* bias, int32_t h, void* out,
+                       int32_t out_bf16, void* stream) {
+  if (n == 0 || h == 0) return PS_OK;
+  if (h > kMaxFirstLayerWidth) return fail(PS_ERR_INVALID, "first layer wider than 8192");
+  const size_t rows = (size_t)2 * 48 * h * (out_bf16 ? 2 : 4);
+  return for_items(
+      n, boards, (cudaStream_t)stream, [&](int i) { return pots[i]; }, [&](int i) { return stacks[i]; },
+      [&](int i0, int k, const ItemMeta& m) {
+        return launch_boundary_first_layer(k, m, base ? base + (size_t)i0 * h : nullptr,
+                                           percard + (size_t)i0 * 52 * h, wcols, bias, h, (char*)out + i0 * rows,
+                                           out_bf16 ? 1 : 0, (cudaStream_t)stream);
+      });
+}
+
 int ps_boundary_first_layer(int32_t n, const uint8_t* boards, const float* pots, const float* stacks,
                             const float* base, const float* percard, const float* wcols, const float* bias, int32_t h,
                             void* out, int32_t out_bf16, void* stream) {
   if (n < 0 || h < 0 || (n > 0 && h > 0 && (!boards || !pots || !stacks || !base || !percard || !wcols || !out)))
     return fail(PS_ERR_INVALID, "bad argument");
-  if (n == 0 || h == 0) return PS_OK;
-  if (h > kMaxFirstLayerWidth) return fail(PS_ERR_INVALID, "first layer wider than 8192");
-  std::vector<uint8_t> hb((size_t)n * 4);
-  for (int i = 0; i < n; ++i) {
-    uint64_t seen = 0;
-    for (int k = 0; k < 4; ++k) {
-      const uint8_t c = boards[4 * i + k];
-      if (c >= 52 || (seen >> c & 1)) return fail(PS_ERR_INVALID, "boards must hold 4 distinct cards below 52");
-      seen |= 1ull << c;
-      hb[4 * i + k] = c;
-    }
-  }
-  cudaStream_t s = (cudaStream_t)stream;
-  const size_t ob = (hb.size() + 15) & ~(size_t)15;
-  StagingLease lease;
-  CU(lease.acquire(ob + 8 * (size_t)n + 16));
-  lease.using_stream(s);
-  char* d = lease.ptr;
-  float* d_pot = (float*)(d + ob);
-  float* d_stack = d_pot + n;
-  CU(cudaMemcpyAsync(d, hb.data(), hb.size(), cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(d_pot, pots, 4 * (size_t)n, cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(d_stack, stacks, 4 * (size_t)n, cudaMemcpyHostToDevice, s));
-  CU(launch_boundary_first_layer(n, (const uint8_t*)d, d_pot, d_stack, base, percard, wcols, bias, h, out,
-                                 out_bf16 ? 1 : 0, s));
-  CU(cudaStreamSynchronize(s));
-  lease.done();
-  return PS_OK;
+  return first_layer(n, boards, pots, stacks, base, percard, wcols, bias, h, out, out_bf16, stream);
+}
+
+int ps_boundary_first_layer_cards(int32_t n, const uint8_t* boards, const float* pots, const float* stacks,
+                                  const float* percard, const float* wcols, const float* bias, int32_t h, void* out,
+                                  int32_t out_bf16, void* stream) {
+  if (n < 0 || h < 0 || (n > 0 && h > 0 && (!boards || !pots || !stacks || !percard || !wcols || !out)))
+    return fail(PS_ERR_INVALID, "bad argument");
+  return first_layer(n, boards, pots, stacks, nullptr, percard, wcols, bias, h, out, out_bf16, stream);
 }
 
 int ps_eval_fixed_strategy(ps_game* G, const float* w0, const float* w1, float* cfv0, float* cfv1) {

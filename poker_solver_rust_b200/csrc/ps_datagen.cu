@@ -473,70 +473,124 @@ cudaError_t launch_river_average_grad(int n, const ItemMeta& meta, const float* 
 //   W x = W_reach [oop|ip] - sum over combos holding r of W_reach[., c] reach[c]
 //         + board / rank one-hot columns + pot, stack, player columns (+ bias)
 // base[i] = W_reach [oop|ip] and percard[i][k] (the sum over the combos
-// holding card k) come from the caller's GEMMs.  One block per item: the
-// river-independent part of the row goes to shared memory, then every
-// (river, column) element is independent and coalesced along the columns;
-// both players' rows come from one read of percard (they differ by the player
-// column).  out [n][2][48][h].
-template <bool BF16>
-__global__ void k_boundary_first_layer(const uint8_t* __restrict__ boards, const float* __restrict__ pots,
-                                       const float* __restrict__ stacks, const float* __restrict__ base,
-                                       const float* __restrict__ percard, const float* __restrict__ wcols,
-                                       const float* __restrict__ bias, int h, void* __restrict__ out) {
-  extern __shared__ float s_c[];  // [h]
+// holding card k) come from the caller's GEMMs; without base it is half the
+// sum of percard over the 52 cards (every combo holds two), in f64.  One block
+// per item, V adjacent columns per thread for all 48 rivers and both players,
+// the river-independent part in registers: bound by the read of percard and
+// the write of the rows.  With an index division per element and one column at
+// a time, 1024 items of 500 columns took 127 us; 57 us now, base included.
+// out [n][2][48][h].
+template <int V>
+struct Cols {
+  float x[V];
+};
+template <int V>
+__device__ __forceinline__ Cols<V> ld_cols(const float* p) {
+  Cols<V> c;
+  if (V == 2) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    c.x[0] = v.x;
+    c.x[V - 1] = v.y;
+  } else {
+    c.x[0] = *p;
+  }
+  return c;
+}
+template <bool BF16, int V>
+__device__ __forceinline__ void st_cols(void* out, size_t at, const float (&v)[V]) {
+  if (BF16) {
+    __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + at;
+    if (V == 2)
+      *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(v[0], v[V - 1]);
+    else
+      *o = __float2bfloat16_rn(v[0]);
+  } else {
+    float* o = static_cast<float*>(out) + at;
+    if (V == 2)
+      *reinterpret_cast<float2*>(o) = make_float2(v[0], v[V - 1]);
+    else
+      *o = v[0];
+  }
+}
+template <bool BF16, int V>
+__global__ void __launch_bounds__(256) k_boundary_first_layer(const __grid_constant__ ItemMeta meta,
+                                                              const float* __restrict__ base,
+                                                              const float* __restrict__ percard,
+                                                              const float* __restrict__ wcols,
+                                                              const float* __restrict__ bias, int h,
+                                                              void* __restrict__ out) {
   __shared__ uint8_t s_river[kRivers];
   const int item = blockIdx.x;
-  const uint8_t* bd = boards + 4 * item;
-  const uint64_t bmask = (1ull << bd[0]) | (1ull << bd[1]) | (1ull << bd[2]) | (1ull << bd[3]);
+  const uint8_t* bd = meta.board[item];
   const unsigned ranks4 = (1u << (bd[0] >> 2)) | (1u << (bd[1] >> 2)) | (1u << (bd[2] >> 2)) | (1u << (bd[3] >> 2));
-  if (threadIdx.x == 0) {
-    int k = 0;
-    for (int c = 0; c < 52; ++c)
-      if (!(bmask >> c & 1)) s_river[k++] = (uint8_t)c;
+  for (int c = threadIdx.x; c < 52; c += blockDim.x) {
+    const int k = river_pos(bd, c);
+    if (k < kRivers) s_river[k] = (uint8_t)c;
   }
-  const float pot = pots[item], stack = stacks[item];
+  __syncthreads();
+  const float pot = meta.a[item], stack = meta.b[item];
   const float total = __fadd_rn(pot, stack);
   const float norm = total > 0.f ? total : 1.f;
   const float fpot = __fdiv_rn(pot, norm), fstack = __fdiv_rn(stack, norm);
-  const float* wpot = wcols + (size_t)(52 + 13) * h;
-  const float* wstack = wpot + h;
-  const float* wplayer = wstack + h;
-  for (int j = threadIdx.x; j < h; j += blockDim.x) {
-    float c = base[(size_t)item * h + j];
-    for (int k = 0; k < 4; ++k) c += wcols[(size_t)bd[k] * h + j];
-    for (int q = 0; q < 13; ++q)
-      if (ranks4 >> q & 1) c += wcols[(size_t)(52 + q) * h + j];
-    s_c[j] = c + fpot * wpot[j] + fstack * wstack[j] + (bias ? bias[j] : 0.f);
-  }
-  __syncthreads();
   const float* pc = percard + (size_t)item * 52 * h;
   const size_t o0 = (size_t)item * 2 * kRivers * h, o1 = o0 + (size_t)kRivers * h;
-  for (int e = threadIdx.x; e < kRivers * h; e += blockDim.x) {
-    const int ri = e / h, j = e - ri * h;
-    const int r = s_river[ri];
-    float v = s_c[j] - pc[(size_t)r * h + j] + wcols[(size_t)r * h + j];
-    if (!(ranks4 >> (r >> 2) & 1)) v += wcols[(size_t)(52 + (r >> 2)) * h + j];
-    const float v1 = v + wplayer[j];
-    if (BF16) {
-      static_cast<__nv_bfloat16*>(out)[o0 + e] = __float2bfloat16_rn(v);
-      static_cast<__nv_bfloat16*>(out)[o1 + e] = __float2bfloat16_rn(v1);
+  for (int j = V * threadIdx.x; j < h; j += V * blockDim.x) {
+    Cols<V> c;
+    if (base) {
+      c = ld_cols<V>(base + (size_t)item * h + j);
     } else {
-      static_cast<float*>(out)[o0 + e] = v;
-      static_cast<float*>(out)[o1 + e] = v1;
+      double t[V] = {};
+#pragma unroll 13
+      for (int k = 0; k < 52; ++k) {
+        const Cols<V> x = ld_cols<V>(pc + (size_t)k * h + j);
+#pragma unroll
+        for (int e = 0; e < V; ++e) t[e] += (double)x.x[e];
+      }
+#pragma unroll
+      for (int e = 0; e < V; ++e) c.x[e] = (float)(0.5 * t[e]);
+    }
+    auto col = [&](int k) { return ld_cols<V>(wcols + (size_t)k * h + j); };
+    auto plus = [&](const Cols<V>& x) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) c.x[e] += x.x[e];
+    };
+#pragma unroll
+    for (int k = 0; k < 4; ++k) plus(col(bd[k]));
+    for (int q = 0; q < 13; ++q)
+      if (ranks4 >> q & 1) plus(col(52 + q));
+    const Cols<V> wpot = col(65), wstack = col(66), wplayer = col(67);
+#pragma unroll
+    for (int e = 0; e < V; ++e)
+      c.x[e] = c.x[e] + fpot * wpot.x[e] + fstack * wstack.x[e] + (bias ? bias[j + e] : 0.f);
+#pragma unroll 4
+    for (int ri = 0; ri < kRivers; ++ri) {
+      const int r = s_river[ri];
+      const Cols<V> x = ld_cols<V>(pc + (size_t)r * h + j), w = col(r), k = col(52 + (r >> 2));
+      const bool fresh = !(ranks4 >> (r >> 2) & 1);  // the river brings a rank the board lacks
+      float v[V], v1[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        v[e] = c.x[e] - x.x[e] + w.x[e];
+        if (fresh) v[e] += k.x[e];
+        v1[e] = v[e] + wplayer.x[e];
+      }
+      st_cols<BF16, V>(out, o0 + (size_t)ri * h + j, v);
+      st_cols<BF16, V>(out, o1 + (size_t)ri * h + j, v1);
     }
   }
 }
 
-cudaError_t launch_boundary_first_layer(int n, const uint8_t* boards, const float* pots, const float* stacks,
-                                        const float* base, const float* percard, const float* wcols,
-                                        const float* bias, int h, void* out, int bf16, cudaStream_t s) {
+cudaError_t launch_boundary_first_layer(int n, const ItemMeta& meta, const float* base, const float* percard,
+                                        const float* wcols, const float* bias, int h, void* out, int bf16,
+                                        cudaStream_t s) {
   if (n <= 0 || h <= 0) return cudaSuccess;
   if (h > kMaxFirstLayerWidth) return cudaErrorInvalidValue;
-  const size_t smem = sizeof(float) * (size_t)h;
-  if (bf16)
-    k_boundary_first_layer<true><<<n, 256, smem, s>>>(boards, pots, stacks, base, percard, wcols, bias, h, out);
-  else
-    k_boundary_first_layer<false><<<n, 256, smem, s>>>(boards, pots, stacks, base, percard, wcols, bias, h, out);
+  // column pairs where every row starts on one
+  const uintptr_t f32 = (uintptr_t)base | (uintptr_t)percard | (uintptr_t)wcols | (bf16 ? 0 : (uintptr_t)out);
+  const bool two = h % 2 == 0 && (f32 & 7) == 0 && ((uintptr_t)out & 3) == 0;
+  auto k = bf16 ? (two ? k_boundary_first_layer<true, 2> : k_boundary_first_layer<true, 1>)
+                : (two ? k_boundary_first_layer<false, 2> : k_boundary_first_layer<false, 1>);
+  k<<<n, 256, 0, s>>>(meta, base, percard, wcols, bias, h, out);
   return cudaGetLastError();
 }
 

@@ -84,15 +84,16 @@ cudaError_t launch_boundary_river_reduce(int n, const ItemMeta& meta, const void
 cudaError_t launch_river_average_grad(int n, const ItemMeta& meta, const float* reach, const float* g, float* gy,
                                       cudaStream_t s);
 // First layer of a boundary network over every input row of
-// launch_boundary_encode without the rows: base [n][h] (weights times the
-// reach rows), percard [n][52][h] (weights times the reach of the combos
-// holding each card), wcols [68][h] (the board, rank, pot, stack and player
-// columns), bias [h] or null; out [n][2][48][h], f32 or bf16; h at most
-// kMaxFirstLayerWidth (its row part stays in shared memory).
+// launch_boundary_encode without the rows, for n <= kMetaItems items (meta.a =
+// pot, meta.b = stack): base [n][h] (weights times the reach rows; null: half
+// the sum of percard), percard [n][52][h] (weights times the reach of the
+// combos holding each card), wcols [68][h] (the board, rank, pot, stack and
+// player columns), bias [h] or null; out [n][2][48][h], f32 or bf16; h at most
+// kMaxFirstLayerWidth.
 constexpr int kMaxFirstLayerWidth = 8192;
-cudaError_t launch_boundary_first_layer(int n, const uint8_t* boards, const float* pots, const float* stacks,
-                                        const float* base, const float* percard, const float* wcols,
-                                        const float* bias, int h, void* out, int bf16, cudaStream_t s);
+cudaError_t launch_boundary_first_layer(int n, const ItemMeta& meta, const float* base, const float* percard,
+                                        const float* wcols, const float* bias, int h, void* out, int bf16,
+                                        cudaStream_t s);
 // Boundary items of a batch (item = (spot, boundary ordinal)) in the 1326-combo
 // layout (card.rs:50-55 index), [items][2][1326], against each spot's hand-order
 // buffers.  which: BC_SET_VALUES gathers `in` into sp.bcfv; BC_REACH / BC_GRAD

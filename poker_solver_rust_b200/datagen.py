@@ -56,22 +56,25 @@ _CARD_COMBOS = {}
 
 
 def _card_combos(device):
-    """[52, 51] combo indices holding each card (card_pair_to_index order)."""
+    """[5304] input rows of a layer that hold each card: for card 0..51, its 51
+    combos (card_pair_to_index order) of the first reach, then of the second."""
     import torch
 
     key = str(device)
     if key not in _CARD_COMBOS:
         idx = [[a * (101 - a) // 2 + b - 1 if a < b else b * (101 - b) // 2 + a - 1 for b in range(52) if b != a]
                for a in range(52)]
-        _CARD_COMBOS[key] = torch.tensor(idx, dtype=torch.int64, device=device)
+        rows = [p * 1326 + i for card in idx for p in range(2) for i in card]
+        _CARD_COMBOS[key] = torch.tensor(rows, dtype=torch.int64, device=device)
     return _CARD_COMBOS[key]
 
 
 def boundary_first_layer(boards, pots, stacks, reach, weight, bias=None, bf16: bool = False):
     """The first Linear layer (weight [h, 2720], bias [h]) of a boundary
     network over every input row of boundary_encode, without writing the rows
-    (ps_boundary_first_layer): [n, 2, 48, h].  One GEMM over the n reach rows
-    and one batched GEMM per card replace the layer's GEMM over 96 n rows."""
+    (ps_boundary_first_layer_cards): [n, 2, 48, h].  One batched GEMM per card
+    (the reach of the combos holding it, times their weights) replaces the
+    layer's GEMM over 96 n rows."""
     import torch
 
     b = np.ascontiguousarray(boards, np.uint8).reshape(-1, 4)
@@ -79,23 +82,23 @@ def boundary_first_layer(boards, pots, stacks, reach, weight, bias=None, bf16: b
     s = np.ascontiguousarray(stacks, np.float32)
     n, h = b.shape[0], weight.shape[0]
     assert reach.is_cuda and tuple(reach.shape) == (n, 2, 1326) and tuple(weight.shape) == (h, 2720)
-    W = weight.detach().float()
-    R = reach.contiguous().float()
-    Wr = W[:, :2652]
-    base = (R.view(n, 2652) @ Wr.t()).contiguous()  # [n, h]
-    idx = _card_combos(R.device)
-    A = R[:, :, idx].permute(2, 0, 1, 3).reshape(52, n, 102)  # reach of the combos holding each card
-    G = Wr.view(h, 2, 1326)[:, :, idx].permute(2, 1, 3, 0).reshape(52, 102, h)
-    percard = torch.bmm(A, G).permute(1, 0, 2).contiguous()  # [n, 52, h]
-    wcols = W[:, 2652:].t().contiguous()  # [68, h]
-    bias_f = None if bias is None else bias.detach().float().contiguous()
-    out = torch.empty((n, 2, 48, h), dtype=torch.bfloat16 if bf16 else torch.float32, device=R.device)
+    out = torch.empty((n, 2, 48, h), dtype=torch.bfloat16 if bf16 else torch.float32, device=reach.device)
     if n == 0:
         return out
+    with torch.no_grad():
+        wt = weight.detach().float().t().contiguous()  # [2720, h]
+        R = reach.contiguous().float()
+        rows = _card_combos(R.device)
+        A = R.view(n, 2652).index_select(1, rows).view(n, 52, 102).transpose(0, 1)
+        G = wt.index_select(0, rows).view(52, 102, h)
+        percard = torch.empty((n, 52, h), dtype=torch.float32, device=R.device)
+        torch.bmm(A, G, out=percard.transpose(0, 1))
+        wcols = wt[2652:]  # [68, h]
+        bias_f = None if bias is None else bias.detach().float().contiguous()
     stream = torch.cuda.current_stream(R.device).cuda_stream
-    N.check(N.lib().ps_boundary_first_layer(
+    N.check(N.lib().ps_boundary_first_layer_cards(
         n, b.ctypes.data_as(C.POINTER(C.c_uint8)), p.ctypes.data_as(C.POINTER(C.c_float)),
-        s.ctypes.data_as(C.POINTER(C.c_float)), C.c_void_p(base.data_ptr()), C.c_void_p(percard.data_ptr()),
+        s.ctypes.data_as(C.POINTER(C.c_float)), C.c_void_p(percard.data_ptr()),
         C.c_void_p(wcols.data_ptr()), C.c_void_p(0 if bias_f is None else bias_f.data_ptr()), h,
         C.c_void_p(out.data_ptr()), int(bf16), C.c_void_p(stream)))
     return out
