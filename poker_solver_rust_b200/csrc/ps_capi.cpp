@@ -754,8 +754,14 @@ struct Batch {
                                                             : std::min(3, (n + dc->nsm - 1) / dc->nsm);
         const int fp = opts && opts->node_parts > 0 ? opts->node_parts : 3;
         if (fl > kMaxFlowLanes || fp > 16) return fail(PS_ERR_INVALID, "flow_spots_per_cta 1..8, node_parts 1..16");
-        const int rc = adopt_flow(fb, opts && opts->scan_buffers > 0 ? opts->scan_buffers : fb / 64, fl, fp,
-                                  opts ? opts->ctas_per_sm : 0);
+        // a class that is already tuned takes its shape at once: adopting the
+        // default first would set the kernel's shared memory twice per batch,
+        // which waits for another batch's running solve
+        std::array<int, 4> known;
+        const int cap = opts ? opts->ctas_per_sm : 0;
+        const int rc = tune && tuned_flow(flow_tune_key(), &known)
+                           ? adopt_flow(known[0], known[1], known[2], known[3], cap)
+                           : adopt_flow(fb, opts && opts->scan_buffers > 0 ? opts->scan_buffers : fb / 64, fl, fp, cap);
         if (rc) return rc;
       }
     }
@@ -909,6 +915,26 @@ struct Batch {
     return PS_OK;
   }
 
+  // The autotuner's class of this batch (device, scan buffers asked for, hand
+  // count, tree size) and the shape already chosen for a class, if any.
+  long flow_tune_key() const {
+    int hs_max = 4;
+    double nodes = 0;
+    for (auto& gp : games) {
+      hs_max = std::max(hs_max, std::max(gp->hs[0], gp->hs[1]));
+      nodes += (double)gp->arena.size();
+    }
+    return (1l << 62) | ((long)dc->device << 40) | ((long)(req_bufs & 0xFF) << 32) | ((long)(hs_max / 64) << 20) |
+           (long)std::min(1 << 19, (int)std::lround(std::log2(1.0 + nodes / (double)games.size()) * 4));
+  }
+  static bool tuned_flow(long key, std::array<int, 4>* shape) {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto it = g_flow_tune.find(key);
+    if (it == g_flow_tune.end()) return false;
+    *shape = it->second;
+    return true;
+  }
+
   // Autotuner of the dataflow shape: times the real solve job (the reference
   // loop with its exploitability checks: one before the first iteration, after
   // the fifth and after the sixth) on a sample of the batch's spots taken
@@ -917,23 +943,9 @@ struct Batch {
   // tree-size class; the state the trials touched is cleared.
   int autotune_flow(const std::vector<int>& order, int cap_ctas) {
     const int n = (int)games.size();
-    int hs_max = 4;
-    double nodes = 0;
-    for (auto& gp : games) {
-      hs_max = std::max(hs_max, std::max(gp->hs[0], gp->hs[1]));
-      nodes += (double)gp->arena.size();
-    }
-    const long key = (1l << 62) | ((long)dc->device << 40) | ((long)(req_bufs & 0xFF) << 32) |
-                     ((long)(hs_max / 64) << 20) |
-                     (long)std::min(1 << 19, (int)std::lround(std::log2(1.0 + nodes / n) * 4));
-    {
-      std::lock_guard<std::mutex> lk(g_tune_mu);
-      auto it = g_flow_tune.find(key);
-      if (it != g_flow_tune.end()) {
-        const auto& c = it->second;
-        return adopt_flow(c[0], c[1], c[2], c[3], cap_ctas);
-      }
-    }
+    const long key = flow_tune_key();
+    std::array<int, 4> known;
+    if (tuned_flow(key, &known)) return adopt_flow(known[0], known[1], known[2], known[3], cap_ctas);
     struct Cand {
       int b, bufs, lanes, parts;
     };
