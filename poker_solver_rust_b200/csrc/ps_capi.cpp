@@ -63,6 +63,7 @@ constexpr int kMaxInstances = 4;  // spots per CTA in lockstep (ps_batch_opts.in
 // single games with at most this many acting hand-edges (sum over decision
 // edges of the actor's hands) run on one thread-block cluster (Batch::build)
 constexpr int64_t kClusterMaxEdgeHands = 131072;
+constexpr size_t kMaxCtaSmem = 227 * 1024;
 constexpr int kFlowMinSpots = 16;  // batches from this size on run the dataflow kernel by default
 std::mutex g_dev_mu;
 std::mutex g_tune_mu;
@@ -762,7 +763,8 @@ struct Batch {
         const int rc = tune && tuned_flow(flow_tune_key(), &known)
                            ? adopt_flow(known[0], known[1], known[2], known[3], cap)
                            : adopt_flow(fb, opts && opts->scan_buffers > 0 ? opts->scan_buffers : fb / 64, fl, fp, cap);
-        if (rc) return rc;
+        if (rc && (sched == PS_SCHED_FLOW || n > dc->nsm)) return rc;
+        if (rc) flow = false;  // its shared memory does not fit (1176 hands): the step-synchronous kernel
       }
     }
     scratch_ctas = std::max(grid * inst_k, flow ? flow_grid * flow_lanes : 0);
@@ -889,6 +891,12 @@ struct Batch {
     pl.bufs = std::max(1, std::min(pl.warps, bufs));
     pl.split = 0;
     occ = flow_occupancy(b, pl);
+    // a request whose lists fit (12 bytes a hand) goes with one buffer less
+    // where the padding of their chunks does not
+    if (occ < 1 && pl.bufs > 1 && (size_t)pl.bufs * (3 * pl.vstride + 8) * 4 + pl.tables + 1024 <= kMaxCtaSmem) {
+      --pl.bufs;
+      occ = flow_occupancy(b, pl);
+    }
     if (occ < 1 || lanes > pl.warps) return false;
     if (cap_ctas > 0) occ = std::min(occ, cap_ctas);
     g = std::max(1, std::min(nspots, dc->nsm * occ));

@@ -54,3 +54,28 @@ def test_adjoint_routes(n):
         out.append((*b.adjoint(cot), b.root_cfvalues_all()))
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("bufs", [0, 23])
+def test_wide_hands(bufs):
+    """The widest spots there are (1176 hands on a flop) at the default shape,
+    and a request of scan buffers whose padding does not fit (one less then)."""
+    rng = np.random.default_rng(3)
+    sp = []
+    for k in range(16):
+        board = [int(x) for x in rng.choice(52, 3 if bufs == 0 else 5, replace=False)]
+        r = spots.uniform_ranges(rng, board)
+        if bufs:
+            for w in r:  # 800 hands: a stride of 832 floats
+                live = np.flatnonzero(w)
+                w[rng.choice(live, len(live) - 800, replace=False)] = 0
+        s = [ps.BetSizeOptions("50%, a", "a")] * 2
+        sp.append((r, board, ps.TreeConfig(initial_state=ps.BoardState.River if bufs else ps.BoardState.Flop,
+                                           starting_pot=60, effective_stack=100, flop_bet_sizes=s, turn_bet_sizes=s,
+                                           river_bet_sizes=s, depth_limit=None if bufs else 0)))
+    out = []
+    for kw in ({"scan_buffers": bufs, "scheduler": 2} if bufs else {}, {"scheduler": STEP}):
+        b = _batch(sp, **kw)
+        b.run_iterations(0, 2, exploitability=True)
+        out.append((b.results()[0], b.root_cfvalues_all()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
