@@ -62,14 +62,35 @@ def _river_average_grad(boards, scale, reach, g):
     return gy
 
 
+def _kernel_takes(*tensors):
+    """Whether a kernel may read these tensors by address: plain f32 memory of
+    one CUDA device that nothing looks through - no batching or other function
+    transform (their wrappers have no storage of their own), no derivative of
+    the result (reverse or forward mode)."""
+    for t in tensors:
+        try:
+            t.untyped_storage()
+        except RuntimeError:
+            return False
+        if not (type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.float32 and t.layout == torch.strided):
+            return False
+        if t.device != tensors[0].device or t.is_neg():
+            return False
+        if torch.is_grad_enabled() and t.requires_grad:
+            return False
+        if torch.autograd.forward_ad.unpack_dual(t).tangent is not None:
+            return False
+    return True
+
+
 class RiverAverage(torch.autograd.Function):
     """The reach-weighted 48-river average (ps_boundary_river_reduce, combo
     layout) as a function of the network outputs y [n, 2, 48, 1326]; reach
     and the scale are constants.  Backward: dB/dy[i,p,r,c] = scale_i *
     W[i,p,r] * keep[i,r,c] / sum_r' W[i,p,r'] keep[i,r',c], where W[i,p,r] is
     the opponent's reach on combos free of river r (gpu_boundary_eval.rs:146-161),
-    in f64: one kernel (ps_river_average_grad) for a plain f32 gradient, the
-    same formula in torch where the gradient itself is differentiated."""
+    in f64: one kernel (ps_river_average_grad) where it may read the gradient
+    and the reach (_kernel_takes), the same formula in torch elsewhere."""
 
     @staticmethod
     def forward(ctx, y, boards, scale, reach):
@@ -84,8 +105,7 @@ class RiverAverage(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (reach,) = ctx.saved_tensors
-        if (type(g) is torch.Tensor and g.is_cuda and g.dtype == reach.dtype == torch.float32
-                and not (torch.is_grad_enabled() and g.requires_grad)):
+        if _kernel_takes(g, reach):
             return _river_average_grad(ctx.boards, ctx.scale, reach, g), None, None, None
         s = torch.as_tensor(ctx.scale, device=g.device)
         keep = river_keep_mask(ctx.boards, g.device).to(torch.float64)  # [n, 48, 1326]
