@@ -163,9 +163,13 @@ __global__ void __launch_bounds__(kReduceThreads) k_boundary_river_reduce(const 
 
 // The average's gradient with respect to the network's outputs, in f64 from
 // f32 inputs: gy[i][p][r][c] = w[r] * (g[i][p][c] * scale / sum of w over the
-// rivers free of c's cards), 0 where the river is one of them.  One block per
-// (item, player), a column pair per thread and round: bound by the write of
-// gy.
+// rivers free of c's cards), where the river is one of them 0 times the
+// bracket: a gradient that is not finite shows there too, as in the formula.
+// One block per (item, player), a column pair per thread and round: bound by
+// the write of gy, which four blocks an SM do fastest (512 items 102 us a call,
+// 107 with the seven that its registers allow, 110 with five and six); the
+// launch asks for kGradPad bytes of shared memory that nothing uses.
+constexpr int kGradPad = 47 * 1024;
 __global__ void __launch_bounds__(kReduceThreads) k_river_average_grad(const __grid_constant__ ItemMeta meta,
                                                             const float* __restrict__ reach,
                                                             const float* __restrict__ g, float* __restrict__ gy,
@@ -182,13 +186,14 @@ __global__ void __launch_bounds__(kReduceThreads) k_river_average_grad(const __g
     const uint64_t ma = blocked_rivers(bd, c), mb = blocked_rivers(bd, c + 1);
     const double da = free_weight(s_w, all, ma), db = free_weight(s_w, all, mb);
     const double ka = da > 0.0 ? (double)gi[c] * scale / da : 0.0, kb = db > 0.0 ? (double)gi[c + 1] * scale / db : 0.0;
+    const float za = (float)(0.0 * ka), zb = (float)(0.0 * kb);
 #pragma unroll 1
     for (int r0 = 0; r0 < kRivers; r0 += 8) {
       const unsigned xa = (unsigned)(ma >> r0), xb = (unsigned)(mb >> r0);
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const double w = s_w[r0 + u];
-        const float2 v = make_float2(xa >> u & 1 ? 0.f : (float)(w * ka), xb >> u & 1 ? 0.f : (float)(w * kb));
+        const float2 v = make_float2(xa >> u & 1 ? za : (float)(w * ka), xb >> u & 1 ? zb : (float)(w * kb));
         float* at = go + (size_t)(r0 + u) * kCombos + c;
         if (pairs) {  // gy is aligned to two values
           *reinterpret_cast<float2*>(at) = v;
@@ -463,7 +468,7 @@ cudaError_t launch_boundary_river_reduce(int n, const ItemMeta& meta, const void
 cudaError_t launch_river_average_grad(int n, const ItemMeta& meta, const float* reach, const float* g, float* gy,
                                       cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_river_average_grad<<<2 * n, kReduceThreads, 0, s>>>(meta, reach, g, gy, ((uintptr_t)gy & 7) == 0);
+  k_river_average_grad<<<2 * n, kReduceThreads, kGradPad, s>>>(meta, reach, g, gy, ((uintptr_t)gy & 7) == 0);
   return cudaGetLastError();
 }
 

@@ -67,16 +67,14 @@ def _kernel_takes(*tensors):
     one CUDA device that nothing looks through - no batching or other function
     transform (their wrappers have no storage of their own), no derivative of
     the result (reverse or forward mode)."""
+    graph, device = torch.is_grad_enabled(), tensors[0].device
     for t in tensors:
+        if not (type(t) is torch.Tensor and t.dtype == torch.float32 and t.is_cuda and t.device == device
+                and t.layout == torch.strided) or t.is_neg() or (graph and t.requires_grad):
+            return False
         try:
-            t.untyped_storage()
+            t.data_ptr()
         except RuntimeError:
-            return False
-        if not (type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.float32 and t.layout == torch.strided):
-            return False
-        if t.device != tensors[0].device or t.is_neg():
-            return False
-        if torch.is_grad_enabled() and t.requires_grad:
             return False
         if torch.autograd.forward_ad.unpack_dual(t).tangent is not None:
             return False

@@ -1,8 +1,9 @@
 """RiverAverage.backward where something looks through the gradient: batched
 gradients, derivatives of the gradient with respect to the reach, forward-mode
-tangents and negative views.  Each is compared with the formula of the backward
-in f64 (within the f32 rounding of the result, 2^-23 relative, and as much for
-the tangents and second derivatives that torch rounds to f32)."""
+tangents, negative views and values that are not finite.  Each is compared with
+the formula of the backward in f64 (within the f32 rounding of the result,
+2^-23 relative, and as much for the tangents and second derivatives that torch
+rounds to f32)."""
 
 import numpy as np
 import pytest
@@ -75,6 +76,17 @@ def test_negative_view():
     g = torch.randn_like(out)
     (got,) = torch.autograd.grad(out, y, torch._neg_view(g))
     _close(got, _formula(boards, scale, reach, -g))
+
+
+def test_non_finite_gradient():
+    """A blocked river's weight is zero times the coefficient, as in the formula."""
+    boards, scale, reach, y = _case(1, seed=4)
+    out = trainer.RiverAverage.apply(y, boards, scale, reach)
+    g = torch.randn_like(out)
+    g[0, 0, ::7], g[0, 1, ::5], g[0, 1, 3::5] = float("inf"), float("nan"), float("-inf")
+    (got,) = torch.autograd.grad(out, y, g)
+    want = _formula(boards, scale, reach, g)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
 
 
 def test_reach_on_another_device_is_refused():
