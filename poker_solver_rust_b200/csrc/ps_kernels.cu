@@ -2199,39 +2199,46 @@ struct SmemLimit {
 static std::mutex g_smem_mu;
 static std::vector<SmemLimit> g_smem_limits;
 
-static cudaError_t set_smem(const void* fn, size_t bytes) {
+static cudaError_t set_smem_locked(const void* fn, size_t bytes) {
   int dev = 0;
   unsigned long long ctx = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = current_context_id(&ctx);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return e;
-  }
-  std::lock_guard<std::mutex> lk(g_smem_mu);
-  SmemLimit* l = nullptr;
-  for (auto& x : g_smem_limits)
-    if (x.fn == fn && x.dev == dev && x.ctx == ctx) l = &x;
-  if (!l || l->bytes != bytes) {
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) {
-      if (l)
-        l->bytes = bytes;
-      else
-        g_smem_limits.push_back(SmemLimit{fn, dev, ctx, bytes});
+  if (e == cudaSuccess) {
+    SmemLimit* l = nullptr;
+    for (auto& x : g_smem_limits)
+      if (x.fn == fn && x.dev == dev && x.ctx == ctx) l = &x;
+    if (!l || l->bytes != bytes) {
+      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      if (e == cudaSuccess) {
+        if (l)
+          l->bytes = bytes;
+        else
+          g_smem_limits.push_back(SmemLimit{fn, dev, ctx, bytes});
+      }
     }
   }
   cudaGetLastError();
   return e;
 }
 
+// Sets the limit and keeps it for its own lifetime, which covers the launch or
+// occupancy query that needs it: the limit is the process's, and a batch of
+// another size built or launched by a second thread would lower it in between
+// (the launch then fails as an invalid argument).
+struct SmemHold {
+  std::lock_guard<std::mutex> lk;
+  cudaError_t e;
+  SmemHold(const void* fn, size_t bytes) : lk(g_smem_mu), e(set_smem_locked(fn, bytes)) {}
+};
+
 size_t setup_smem_bytes() { return sizeof(SetupSmem); }
 
 cudaError_t launch_setup(const SpotDev* spots, const int2* work, int nwork, const int32_t* table, int* err,
                          int grid, cudaStream_t s) {
   size_t sm = sizeof(SetupSmem);
-  cudaError_t e = set_smem((const void*)k_setup, sm);
-  if (e != cudaSuccess) return e;
+  SmemHold hold((const void*)k_setup, sm);
+  if (hold.e != cudaSuccess) return hold.e;
   k_setup<<<grid, 512, sm, s>>>(spots, work, nwork, table, err);
   return cudaGetLastError();
 }
@@ -2245,8 +2252,8 @@ cudaError_t launch_solve(const SpotDev* spots, int ninst, int K, const int* inst
     return cudaErrorInvalidValue;
   size_t smem = plan.total();
   const void* fn = plan.split ? (const void*)k_solve<true> : (const void*)k_solve<false>;
-  cudaError_t e = set_smem(fn, smem);
-  if (e != cudaSuccess) return e;
+  SmemHold hold(fn, smem);
+  if (hold.e != cudaSuccess) return hold.e;
   if (plan.split)
     k_solve<true><<<grid, block, smem, s>>>(spots, ninst, K, inst, counter, disc, job, target, scratch, scratch_floats,
                                      out_expl, out_iters, plan, err);
@@ -2272,8 +2279,8 @@ cudaError_t launch_flow(const SpotDev* spots, int ninst, const int* inst, int* c
     return cudaErrorInvalidValue;
   size_t smem = plan.total();
   const int kind = job.adjoint ? FLOW_ADJOINT : boundaries ? FLOW_BOUNDARY : FLOW_PLAIN;
-  cudaError_t e = set_smem(flow_kernel(kind), smem);
-  if (e != cudaSuccess) return e;
+  SmemHold hold(flow_kernel(kind), smem);
+  if (hold.e != cudaSuccess) return hold.e;
   FlowArgs A{spots, ninst, inst, counter, disc, job, target, scratch, scratch_floats, out_expl, out_iters, err,
              lanes, node_parts};
   SmemPlan pl = plan;
@@ -2281,16 +2288,16 @@ cudaError_t launch_flow(const SpotDev* spots, int ninst, const int* inst, int* c
   return cudaLaunchKernel(flow_kernel(kind), dim3(grid), dim3(block), args, smem, s);
 }
 
-int flow_occupancy(int block, const SmemPlan& plan) {
+int flow_occupancy(int block, const SmemPlan& plan, bool boundaries) {
+  // the instantiation that the batch's solves run; the adjoint's has the same
+  // launch bounds and static shared memory
+  const void* fn = flow_kernel(boundaries ? FLOW_BOUNDARY : FLOW_PLAIN);
   size_t smem = plan.total();
-  int least = 1 << 30;  // the launch shape serves every job of the batch
-  for (int kind : {FLOW_PLAIN, FLOW_BOUNDARY, FLOW_ADJOINT}) {
-    int n = 0;
-    if (set_smem(flow_kernel(kind), smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, flow_kernel(kind), block, smem) != cudaSuccess) return 0;
-    least = n < least ? n : least;
-  }
-  return least;
+  SmemHold hold(fn, smem);
+  int n = 0;
+  if (hold.e != cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) != cudaSuccess)
+    return 0;
+  return n;
 }
 
 int grid_ctas(int block, const SmemPlan& plan) {
@@ -2298,7 +2305,8 @@ int grid_ctas(int block, const SmemPlan& plan) {
   size_t smem = plan.total();
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (set_smem((const void*)k_grid, smem) != cudaSuccess) return 0;
+  SmemHold hold((const void*)k_grid, smem);
+  if (hold.e != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_grid, block, smem) != cudaSuccess) return 0;
   return nsm * per_sm;
 }
@@ -2311,7 +2319,8 @@ static cudaError_t grid_cluster_attrs() {
 int grid_cluster_fits(int ctas, int block, const SmemPlan& plan) {
   if (ctas < 2 || ctas > 16) return 0;
   const size_t smem = plan.total();
-  if (set_smem((const void*)k_grid, smem) != cudaSuccess || grid_cluster_attrs() != cudaSuccess) return 0;
+  SmemHold hold((const void*)k_grid, smem);
+  if (hold.e != cudaSuccess || grid_cluster_attrs() != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -2335,9 +2344,9 @@ cudaError_t launch_grid(const SpotDev* spot, const GridJob& job, const Discount*
                         size_t scratch_floats, float* out_expl, int* out_iters, unsigned* bar, double* gred,
                         int* err, int grid, int block, const SmemPlan& plan, cudaStream_t s, int cluster) {
   size_t smem = plan.total();
-  cudaError_t e = set_smem((const void*)k_grid, smem);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(bar, 0, 4 * sizeof(unsigned), s);  // count, generation, abort word
+  SmemHold hold((const void*)k_grid, smem);
+  if (hold.e != cudaSuccess) return hold.e;
+  cudaError_t e = cudaMemsetAsync(bar, 0, 4 * sizeof(unsigned), s);  // count, generation, abort word
   if (e != cudaSuccess) return e;
   GridJob j = job;
   j.cluster = cluster ? 1 : 0;
@@ -2366,8 +2375,8 @@ cudaError_t launch_iterate(const SpotDev* spots, int nspots, const Discount* dis
                            size_t scratch_floats, int* err, int grid, int block, const SmemPlan& plan,
                            cudaStream_t s) {
   size_t smem = plan.total();
-  cudaError_t e = set_smem((const void*)k_iterate, smem);
-  if (e != cudaSuccess) return e;
+  SmemHold hold((const void*)k_iterate, smem);
+  if (hold.e != cudaSuccess) return hold.e;
   k_iterate<<<grid, block, smem, s>>>(spots, nspots, disc, t0, t1, scratch, scratch_floats, plan, err);
   return cudaGetLastError();
 }
@@ -2375,8 +2384,8 @@ cudaError_t launch_iterate(const SpotDev* spots, int nspots, const Discount* dis
 cudaError_t launch_exploitability(const SpotDev* spots, int nspots, float* scratch, size_t scratch_floats,
                                   float* out, int* err, int grid, int block, const SmemPlan& plan, cudaStream_t s) {
   size_t smem = plan.total();
-  cudaError_t e = set_smem((const void*)k_exploitability, smem);
-  if (e != cudaSuccess) return e;
+  SmemHold hold((const void*)k_exploitability, smem);
+  if (hold.e != cudaSuccess) return hold.e;
   k_exploitability<<<grid, block, smem, s>>>(spots, nspots, scratch, scratch_floats, out, plan, err);
   return cudaGetLastError();
 }
@@ -2385,8 +2394,8 @@ cudaError_t launch_average(const SpotDev* spots, int nspots, int save, int playe
                            float* scratch, size_t scratch_floats, float* out, int* err, int grid, int block,
                            const SmemPlan& plan, cudaStream_t s, int owner, float* bgrad, float* breach) {
   size_t smem = plan.total();
-  cudaError_t e = set_smem((const void*)k_average, smem);
-  if (e != cudaSuccess) return e;
+  SmemHold hold((const void*)k_average, smem);
+  if (hold.e != cudaSuccess) return hold.e;
   k_average<<<grid, block, smem, s>>>(spots, nspots, save, player, root_reach, scratch, scratch_floats, out, owner,
                                        bgrad, breach, plan,
                                        err);
@@ -2396,8 +2405,8 @@ cudaError_t launch_average(const SpotDev* spots, int nspots, int save, int playe
 cudaError_t launch_eval_terminal(const SpotDev* spots, Op op, int player, float* scratch, size_t scratch_floats,
                                  int* err, int block, const SmemPlan& plan, cudaStream_t s) {
   size_t smem = plan.total();
-  cudaError_t e = set_smem((const void*)k_eval_terminal, smem);
-  if (e != cudaSuccess) return e;
+  SmemHold hold((const void*)k_eval_terminal, smem);
+  if (hold.e != cudaSuccess) return hold.e;
   k_eval_terminal<<<1, block, smem, s>>>(spots, op, player, scratch, scratch_floats, plan, err);
   return cudaGetLastError();
 }
@@ -2489,11 +2498,13 @@ cudaError_t launch_exploitability_fixed(const SpotDev* spot, size_t slot_floats,
   e = cudaMemsetAsync(base, 0, kFixedScratchHeader * sizeof(float), s);
   if (e != cudaSuccess) return e;
   size_t smem = plan.total();
-  e = set_smem((const void*)k_exploitability, smem);
-  if (e != cudaSuccess) return e;
-  k_exploitability<<<1, block, smem, s>>>(spot, 1, base + kFixedScratchHeader, slot_floats, base, plan,
-                                          reinterpret_cast<int*>(base + 1));
-  e = cudaGetLastError();
+  {
+    SmemHold hold((const void*)k_exploitability, smem);
+    if (hold.e != cudaSuccess) return hold.e;
+    k_exploitability<<<1, block, smem, s>>>(spot, 1, base + kFixedScratchHeader, slot_floats, base, plan,
+                                            reinterpret_cast<int*>(base + 1));
+    e = cudaGetLastError();
+  }
   if (e != cudaSuccess) return e;
   float head[2];
   e = cudaMemcpyAsync(head, base, sizeof(head), cudaMemcpyDeviceToHost, s);
@@ -2552,7 +2563,7 @@ extern "C" int ps_debug_phase_cycles(unsigned long long* out, int n) {
 int solve_occupancy(int block, const SmemPlan& plan) {
   int n = 0;
   size_t smem = plan.total();
-  set_smem((const void*)k_solve<false>, smem);
+  SmemHold hold((const void*)k_solve<false>, smem);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_solve<false>, block, smem) != cudaSuccess) return 1;
   return n < 1 ? 1 : n;
 }

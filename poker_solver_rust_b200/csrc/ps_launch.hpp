@@ -193,7 +193,7 @@ cudaError_t launch_flow(const SpotDev* spots, int ninst, const int* inst, int* c
                         const SolveJob& job, const float* target, float* scratch, size_t scratch_floats,
                         float* out_expl, int* out_iters, int* err, int grid, int block, int lanes, int node_parts,
                         const SmemPlan& plan, cudaStream_t s, bool boundaries);
-int flow_occupancy(int block, const SmemPlan& plan);  // CTAs per SM (0 = does not fit)
+int flow_occupancy(int block, const SmemPlan& plan, bool boundaries);  // CTAs per SM (0 = does not fit)
 cudaError_t launch_iterate(const SpotDev* spots, int nspots, const Discount* disc, int t0, int t1,
                            float* scratch, size_t scratch_floats, int* err, int grid, int block,
                            const SmemPlan& plan, cudaStream_t s);

@@ -1,0 +1,82 @@
+"""Launch requests of a batch: what may be asked for, what it costs and what is
+shared between batches (tuned shapes, a kernel's shared-memory limit)."""
+
+import threading
+
+import numpy as np
+import pytest
+
+import poker_solver_rust_b200 as ps
+from tests import spots
+
+pytestmark = pytest.mark.gpu
+
+STEP, FLOW = 1, 2
+
+
+def _thin(n, seed, hands=90, stack=200):
+    """River spots of one tree with `hands` hands a player."""
+    rng = np.random.default_rng(seed)
+    sizes = ps.BetSizeOptions("50%, a", "100%, a")
+    t = ps.TreeConfig(initial_state=ps.BoardState.River, starting_pot=100, effective_stack=stack,
+                      river_bet_sizes=[sizes, sizes])
+    sp = []
+    for _ in range(n):
+        board = [int(x) for x in rng.choice(52, 5, replace=False)]
+        r = np.zeros((2, 1326), np.float32)
+        for w in r:
+            live = rng.permutation(np.flatnonzero(~spots._board_blocked(board)))[:hands]
+            w[live] = rng.random(hands).astype(np.float32) * 0.9 + 0.1
+        sp.append((r, board, t))
+    return sp
+
+
+def _batch(sp, **kw):
+    return ps.BatchSolver([spots.card_config(r, b) for r, b, _ in sp], [t for _, _, t in sp], **kw)
+
+
+def _solved(b, iterations=20):
+    b.solve(iterations, 0.01 * b.starting_pots)
+    return (*b.results(), b.root_cfvalues_all())
+
+
+def _same(a, b):
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
+
+
+def test_batches_of_different_sizes_launch_from_several_threads():
+    """Each launch sets its kernel's shared-memory limit; another thread's batch of another stride must
+    not change it before the launch."""
+    batches = [_batch(_thin(16, seed=k, hands=40 + 120 * k)) for k in range(4)]
+    want = []
+    for b in batches:
+        assert b.config()["scheduler"] == "dataflow"
+        b.run_iterations(0, 2, root=True)
+        want.append(b.root_cfvalues_all())
+    errors = []
+
+    def launch(b):
+        try:
+            for _ in range(400):
+                if errors:
+                    return
+                b.run_iterations(2, 2, root=True)
+        except Exception as e:
+            errors.append(e)
+
+    def build():
+        try:
+            for k in range(40):
+                _batch(_thin(16, seed=k, hands=30 + 64 * (k % 5)))
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=launch, args=(b,)) for b in batches] + [threading.Thread(target=build)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for b, w in zip(batches, want):
+        assert np.array_equal(b.root_cfvalues_all(), w)
