@@ -754,17 +754,25 @@ struct Batch {
         const int fl = opts && opts->flow_spots_per_cta > 0 ? opts->flow_spots_per_cta
                                                             : std::min(3, (n + dc->nsm - 1) / dc->nsm);
         const int fp = opts && opts->node_parts > 0 ? opts->node_parts : 3;
-        if (fl > kMaxFlowLanes || fp > 16) return fail(PS_ERR_INVALID, "flow_spots_per_cta 1..8, node_parts 1..16");
-        // a class that is already tuned takes its shape at once: adopting the
-        // default first would set the kernel's shared memory twice per batch,
-        // which waits for another batch's running solve
-        std::array<int, 4> known;
-        const int cap = opts ? opts->ctas_per_sm : 0;
-        const int rc = tune && tuned_flow(flow_tune_key(), &known)
-                           ? adopt_flow(known[0], known[1], known[2], known[3], cap)
-                           : adopt_flow(fb, opts && opts->scan_buffers > 0 ? opts->scan_buffers : fb / 64, fl, fp, cap);
-        if (rc && (sched == PS_SCHED_FLOW || n > dc->nsm)) return rc;
-        if (rc) flow = false;  // its shared memory does not fit (1176 hands): the step-synchronous kernel
+        // a batch that ran step-synchronously whatever its dataflow request
+        // said does so where the request is out of range or its shared memory
+        // does not fit (scan_buffers = 32 with 1081 hands)
+        const bool must = sched == PS_SCHED_FLOW || n > dc->nsm;
+        if (fl > kMaxFlowLanes || fp > 16) {
+          if (must) return fail(PS_ERR_INVALID, "flow_spots_per_cta 1..8, node_parts 1..16");
+          flow = false;
+        } else {
+          // a class that is already tuned takes its shape at once: adopting the
+          // default first would set the kernel's shared memory twice per batch,
+          // which waits for another batch's running solve
+          std::array<int, 4> known;
+          const int cap = opts ? opts->ctas_per_sm : 0;
+          const int rc = tune && tuned_flow(flow_tune_key(), &known)
+                             ? adopt_flow(known[0], known[1], known[2], known[3], cap)
+                             : adopt_flow(fb, opts && opts->scan_buffers > 0 ? opts->scan_buffers : fb / 64, fl, fp, cap);
+          if (rc && must) return rc;
+          if (rc) flow = false;
+        }
       }
     }
     scratch_ctas = std::max(grid * inst_k, flow ? flow_grid * flow_lanes : 0);

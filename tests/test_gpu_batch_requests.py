@@ -80,3 +80,16 @@ def test_batches_of_different_sizes_launch_from_several_threads():
     assert not errors, errors
     for b, w in zip(batches, want):
         assert np.array_equal(b.root_cfvalues_all(), w)
+
+
+@pytest.mark.parametrize("request_", [{"flow_spots_per_cta": 9}, {"node_parts": 17}, {"scan_buffers": 32}])
+def test_small_batch_ignores_a_dataflow_request_it_cannot_run(request_):
+    """Up to a spot per SM the default schedule takes any dataflow request; more spots, or the dataflow
+    scheduler asked for, refuse one that is out of range."""
+    sp = _thin(16, seed=3, hands=1000)
+    b = _batch(sp, **request_)
+    assert b.config()["scheduler"] == "step-synchronous"
+    _same(_solved(b), _solved(_batch(sp, scheduler=STEP)))
+    for kw in ({"scheduler": FLOW}, {}):
+        with pytest.raises(Exception):
+            _batch(sp if kw else _thin(150, seed=3, hands=1000), **request_, **kw)
