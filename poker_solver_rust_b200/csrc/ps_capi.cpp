@@ -898,10 +898,11 @@ struct Batch {
     pl.warps = b / 32;
     pl.bufs = std::max(1, std::min(pl.warps, bufs));
     pl.split = 0;
+    pl.tables = 0;  // k_flow reads the board tables from global memory, also where staging was asked for
     occ = flow_occupancy(b, pl, !items.empty());
     // a request whose lists fit (12 bytes a hand) goes with one buffer less
     // where the padding of their chunks does not
-    if (occ < 1 && pl.bufs > 1 && (size_t)pl.bufs * (3 * pl.vstride + 8) * 4 + pl.tables + 1024 <= kMaxCtaSmem) {
+    if (occ < 1 && pl.bufs > 1 && (size_t)pl.bufs * (3 * pl.vstride + 8) * 4 + 1024 <= kMaxCtaSmem) {
       --pl.bufs;
       occ = flow_occupancy(b, pl, !items.empty());
     }

@@ -93,3 +93,12 @@ def test_small_batch_ignores_a_dataflow_request_it_cannot_run(request_):
     for kw in ({"scheduler": FLOW}, {}):
         with pytest.raises(Exception):
             _batch(sp if kw else _thin(150, seed=3, hands=1000), **request_, **kw)
+
+
+def test_dataflow_with_staged_tables_asked_for():
+    """13 scan buffers of 1080 hands and a request to stage the board tables: the dataflow kernel reads
+    the tables from global memory, so only the buffers count."""
+    sp = _thin(150, seed=4, hands=1080)
+    b = _batch(sp, stage_tables=1, scan_buffers=13)
+    assert b.config()["scheduler"] == "dataflow" and b.config()["scan_buffers"] == 13
+    _same(_solved(b, 5), _solved(_batch(sp, scheduler=STEP), 5))
