@@ -775,7 +775,7 @@ struct Batch {
         }
       }
     }
-    scratch_ctas = std::max(grid * inst_k, flow ? flow_grid * flow_lanes : 0);
+    scratch_ctas = std::max(grid * inst_k, flow ? flow_scratch(flow_grid, flow_lanes, n) : 0);
     CU(dalloc(&d_scratch, sizeof(float) * scratch_floats * scratch_ctas));
     // a single tree of at least PS_GRID_NODES nodes (default 16; 0 = never)
     // is solved by all SMs at once: a lone game is latency-bound, and even a
@@ -912,16 +912,21 @@ struct Batch {
     return true;
   }
 
+  // Scratch areas of a launch: one per lane that finds a spot (k_flow numbers
+  // them by the lanes' first queue places).
+  static int flow_scratch(int g, int lanes, int nspots) { return std::min(nspots, g * lanes); }
+
   int adopt_flow(int b, int bufs, int lanes, int parts, int cap_ctas) {
     SmemPlan pl;
     int occ, g;
     if (!flow_shape(b, bufs, lanes, cap_ctas, (int)games.size(), pl, occ, g))
       return fail(PS_ERR_INVALID, "dataflow launch shape does not fit: " + std::to_string(b) + " threads, " +
                                       std::to_string(bufs) + " scan buffers, " + std::to_string(lanes) + " spots");
-    if (d_scratch && (size_t)g * lanes > (size_t)scratch_ctas) {
+    const int places = flow_scratch(g, lanes, (int)games.size());
+    if (d_scratch && places > scratch_ctas) {
       dfree(d_scratch);
-      CU(dalloc(&d_scratch, sizeof(float) * scratch_floats * g * lanes));
-      scratch_ctas = g * lanes;
+      CU(dalloc(&d_scratch, sizeof(float) * scratch_floats * places));
+      scratch_ctas = places;
     }
     flow_block = b;
     flow_plan = pl;
@@ -1009,7 +1014,7 @@ struct Batch {
       SmemPlan pl;
       int occ, g;
       if (flow_shape(c.b, c.bufs, c.lanes, cap_ctas, ns, pl, occ, g))
-        max_scr = std::max(max_scr, (size_t)g * c.lanes);
+        max_scr = std::max(max_scr, (size_t)flow_scratch(g, c.lanes, ns));
     }
     char* tmp = nullptr;
     const size_t tb = align256(sizeof(SpotDev) * ns) + align256(20 * (size_t)ns) + 256;
@@ -1112,6 +1117,7 @@ struct Batch {
     }
     size_t max_scr = (size_t)ns;
     ns = std::min(n, 4 * ns);
+    max_scr = std::min(max_scr, (size_t)ns);
     std::vector<SpotDev> sample(ns);
     std::vector<int> ids(ns);
     std::vector<float> tg(ns);

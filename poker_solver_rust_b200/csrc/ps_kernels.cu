@@ -1741,8 +1741,8 @@ __global__ void __launch_bounds__(kMaxFlowBlock, 1) k_flow(FlowArgs A, SmemPlan 
       // cost, so every CTA starts with spots of about the same total (bound
       // as the warps came, the first CTAs took the costliest spots each)
       const int b = warp & 1 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
-      bound = lane_bind(L, A, A.scratch + ((size_t)blockIdx.x * K + warp) * A.scratch_floats, plan,
-                        warp * (int)gridDim.x + b);
+      const int place = warp * (int)gridDim.x + b;  // also the lane's scratch area: only lanes with a spot have one
+      bound = lane_bind(L, A, A.scratch + (size_t)place * A.scratch_floats, plan, place);
       if (!bound) atomicAdd(&s_retired, 1);
     }
     if (__shfl_sync(0xffffffffu, bound, 0) && lane_move(L, A, plan) && lane == 0) atomicAdd(&s_retired, 1);

@@ -184,9 +184,10 @@ cudaError_t launch_solve(const SpotDev* spots, int ninst, int K, const int* inst
 // Dataflow batched solve (k_flow): each CTA holds `lanes` spots at once, each
 // at its own step; warps claim the steps' items (terminal runs; node ops cut
 // into node_parts column blocks) instead of waiting at per-step barriers.
-// The same jobs as launch_solve (boundaries: some spot has depth boundaries); inst: [ninst] spot ids in
-// the order they are handed out; scratch holds lanes * scratch_floats floats
-// per CTA.  Results equal launch_solve's bit for bit.
+// The same jobs as launch_solve (boundaries: some spot has depth boundaries);
+// inst: [ninst] spot ids in the order they are handed out; scratch holds an
+// area of scratch_floats floats for each of the min(ninst, lanes * grid) lanes
+// that start with a spot.  Results equal launch_solve's bit for bit.
 constexpr int kMaxFlowThreads = 1024;
 constexpr int kMaxFlowLanes = 8;
 cudaError_t launch_flow(const SpotDev* spots, int ninst, const int* inst, int* counter, const Discount* disc,

@@ -1,6 +1,8 @@
 """Launch requests of a batch: what may be asked for, what it costs and what is
 shared between batches (tuned shapes, a kernel's shared-memory limit)."""
 
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -102,3 +104,26 @@ def test_dataflow_with_staged_tables_asked_for():
     b = _batch(sp, stage_tables=1, scan_buffers=13)
     assert b.config()["scheduler"] == "dataflow" and b.config()["scan_buffers"] == 13
     _same(_solved(b, 5), _solved(_batch(sp, scheduler=STEP), 5))
+
+
+_SCRATCH = """
+import torch
+from tests.test_gpu_batch_requests import _batch, _thin
+free = lambda: torch.cuda.mem_get_info()[0]
+sp = _thin(149, seed=5, hands=1080, stack=2000)
+at, used, keep = free(), [], []
+for lanes in (1, 8):
+    keep.append(_batch(sp, scheduler=2, flow_spots_per_cta=lanes, scan_buffers=8))
+    used.append(at - free())
+    at -= used[-1]
+print("BYTES", *used)
+"""
+
+
+def test_scratch_is_for_spots_not_for_idle_lanes():
+    """149 spots take 149 scratch areas whether a CTA may hold one spot or eight (in a process of its
+    own, where no freed memory waits in the library's pool)."""
+    r = subprocess.run([sys.executable, "-c", _SCRATCH], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    one, eight = [int(x) for x in r.stdout.split("BYTES")[1].split()]
+    assert eight <= one + (64 << 20), (one, eight)
