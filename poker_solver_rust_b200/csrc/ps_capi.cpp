@@ -64,6 +64,7 @@ constexpr int kMaxInstances = 4;  // spots per CTA in lockstep (ps_batch_opts.in
 // edges of the actor's hands) run on one thread-block cluster (Batch::build)
 constexpr int64_t kClusterMaxEdgeHands = 131072;
 constexpr size_t kMaxCtaSmem = 227 * 1024;
+constexpr int kMaxTunedLanes = 4;  // spots per CTA that the dataflow autotuner tries
 constexpr int kFlowMinSpots = 16;  // batches from this size on run the dataflow kernel by default
 std::mutex g_dev_mu;
 std::mutex g_tune_mu;
@@ -304,8 +305,8 @@ struct StagingLease {
 std::map<long, std::pair<int, int>> g_tune;  // autotuned (CTA size, scan-buffer warps) per
                                              // (device, hand-count class, tree-size class)
 DeviceConsts g_dev[16];
-std::map<long, std::array<int, 4>> g_flow_tune;  // autotuned dataflow shape (threads, scan buffers, spots per
-                                                 // CTA, node parts) per (device, hand-count, tree-size class)
+std::map<long, std::array<int, 4>> g_flow_tune;  // autotuned dataflow shape (threads, scan buffers, spots per CTA,
+                                                 // node parts) per class (Batch::flow_tune_key)
 
 int device_consts(DeviceConsts** out) {
   int dev = 0;
@@ -767,11 +768,12 @@ struct Batch {
           // which waits for another batch's running solve
           std::array<int, 4> known;
           const int cap = opts ? opts->ctas_per_sm : 0;
-          const int rc = tune && tuned_flow(flow_tune_key(), &known)
-                             ? adopt_flow(known[0], known[1], known[2], known[3], cap)
-                             : adopt_flow(fb, opts && opts->scan_buffers > 0 ? opts->scan_buffers : fb / 64, fl, fp, cap);
-          if (rc && must) return rc;
-          if (rc) flow = false;
+          if (!(tune && tuned_flow(flow_tune_key(), &known) &&
+                adopt_flow(known[0], known[1], known[2], known[3], cap) == PS_OK)) {
+            const int rc = adopt_flow(fb, opts && opts->scan_buffers > 0 ? opts->scan_buffers : fb / 64, fl, fp, cap);
+            if (rc && must) return rc;
+            if (rc) flow = false;
+          }
         }
       }
     }
@@ -937,8 +939,12 @@ struct Batch {
     return PS_OK;
   }
 
-  // The autotuner's class of this batch (device, scan buffers asked for, hand
-  // count, tree size) and the shape already chosen for a class, if any.
+  // The autotuner's class of this batch (device, scan buffers asked for, spots
+  // per SM, hand count, tree size) and the shape already chosen for a class, if
+  // any.  Spots per SM up to one more than the most that is tried: a batch of
+  // one or two runs alike with any number of spots per CTA (301 river spots
+  // 67-68 ms with 1, 2 or 3), so its choice says nothing for a larger one (1500
+  // spots 273 ms with 1, 154 with 3).
   long flow_tune_key() const {
     int hs_max = 4;
     double nodes = 0;
@@ -946,7 +952,9 @@ struct Batch {
       hs_max = std::max(hs_max, std::max(gp->hs[0], gp->hs[1]));
       nodes += (double)gp->arena.size();
     }
-    return (1l << 62) | ((long)dc->device << 40) | ((long)(req_bufs & 0xFF) << 32) | ((long)(hs_max / 64) << 20) |
+    const long per_sm = std::min(kMaxTunedLanes + 1, ((int)games.size() + dc->nsm - 1) / dc->nsm);
+    return (1l << 62) | (per_sm << 48) | ((long)dc->device << 40) | ((long)(req_bufs & 0xFF) << 32) |
+           ((long)(hs_max / 64) << 20) |
            (long)std::min(1 << 19, (int)std::lround(std::log2(1.0 + nodes / (double)games.size()) * 4));
   }
   static bool tuned_flow(long key, std::array<int, 4>* shape) {
@@ -967,13 +975,14 @@ struct Batch {
     const int n = (int)games.size();
     const long key = flow_tune_key();
     std::array<int, 4> known;
-    if (tuned_flow(key, &known)) return adopt_flow(known[0], known[1], known[2], known[3], cap_ctas);
+    // (a shape of this class that does not fit this batch's slot stride: tuned anew)
+    if (tuned_flow(key, &known) && adopt_flow(known[0], known[1], known[2], known[3], cap_ctas) == PS_OK) return PS_OK;
     struct Cand {
       int b, bufs, lanes, parts;
     };
     std::vector<Cand> cands;
     for (int b : {256, 512, 1024})
-      for (int lanes : {1, 2, 3, 4})
+      for (int lanes = 1; lanes <= kMaxTunedLanes; ++lanes)
         for (int parts : {1, 2, 3}) {
           const int w = b / 32;
           if (req_bufs > 0) {

@@ -127,3 +127,22 @@ def test_scratch_is_for_spots_not_for_idle_lanes():
     assert r.returncode == 0, r.stderr
     one, eight = [int(x) for x in r.stdout.split("BYTES")[1].split()]
     assert eight <= one + (64 << 20), (one, eight)
+
+
+def test_shapes_are_tuned_per_batch_size():
+    """A shape tuned on little more than a spot per SM is not adopted for many spots per SM."""
+    sp = _thin(900, seed=71, hands=212)
+    _solved(_batch(sp[:200], block_threads=-1), 5)
+    large = _batch(sp, block_threads=-1)
+    assert large.autotune_trials()
+    _solved(large, 5)
+    assert not _batch(sp[:820], block_threads=-1).autotune_trials()  # the same class: no trials
+
+
+def test_tuned_shape_that_does_not_fit_is_replaced():
+    """576 and 608 hands are one hand-count class, and 32 scan buffers fit in shared memory for the
+    first only: whatever was tuned for the first, the second is built and solved."""
+    for hands in (576, 608):
+        sp = _thin(200, seed=72, hands=hands)
+        b = _batch(sp, block_threads=-1)
+        _same(_solved(b, 10), _solved(_batch(sp, scheduler=STEP), 10))
