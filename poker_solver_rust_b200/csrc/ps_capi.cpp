@@ -92,7 +92,9 @@ struct PinnedPool {
   };
   std::mutex mu;
   std::vector<Buf> free_;
-  cudaError_t acquire(size_t bytes, char** out, CtxTag* tag) {
+  // A block of at least *bytes; *bytes becomes its size, which release() takes
+  // back.  The smallest kept block that is large enough.
+  cudaError_t acquire(size_t* bytes, char** out, CtxTag* tag) {
     cudaError_t e = current_tag(tag);
     if (e != cudaSuccess) return e;
     {
@@ -100,14 +102,17 @@ struct PinnedPool {
       free_.erase(std::remove_if(free_.begin(), free_.end(),
                                  [&](const Buf& b) { return b.tag.dev == tag->dev && b.tag.ctx != tag->ctx; }),
                   free_.end());
-      for (size_t i = 0; i < free_.size(); ++i)
-        if (free_[i].bytes >= bytes && free_[i].tag.ctx == tag->ctx) {
-          *out = free_[i].p;
-          free_.erase(free_.begin() + (long)i);
-          return cudaSuccess;
-        }
+      auto best = free_.end();
+      for (auto it = free_.begin(); it != free_.end(); ++it)
+        if (it->bytes >= *bytes && it->tag.ctx == tag->ctx && (best == free_.end() || it->bytes < best->bytes)) best = it;
+      if (best != free_.end()) {
+        *out = best->p;
+        *bytes = best->bytes;
+        free_.erase(best);
+        return cudaSuccess;
+      }
     }
-    return cudaMallocHost(out, bytes);
+    return cudaMallocHost(out, *bytes);
   }
   void release(char* p, size_t bytes, const CtxTag& tag) {
     std::lock_guard<std::mutex> lk(mu);
@@ -120,7 +125,8 @@ struct PinnedPool {
     }
   }
 };
-PinnedPool g_pinned;
+PinnedPool g_pinned;       // batch uploads
+PinnedPool g_copy_blocks;  // copy_out, at most 32 MB each: they neither take nor push out a batch's block
 
 // Streams and their four timing events, kept for reuse by the next batch:
 // creating a stream or an event waits while a kernel of another batch runs
@@ -196,7 +202,8 @@ cudaError_t copy_out(void* dst, const void* src, size_t bytes, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   char* pin = nullptr;
   CtxTag tag;
-  if (nt < 2 || g_pinned.acquire(nt * kPiece, &pin, &tag) != cudaSuccess) {
+  size_t pinned = nt * kPiece;
+  if (nt < 2 || g_copy_blocks.acquire(&pinned, &pin, &tag) != cudaSuccess) {
     cudaGetLastError();  // no pinned memory: the plain copy
     e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
     return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
@@ -222,7 +229,7 @@ cudaError_t copy_out(void* dst, const void* src, size_t bytes, cudaStream_t s) {
   for (cudaError_t x : err)
     if (x != cudaSuccess) e = x;
   cudaStreamSynchronize(s);  // no piece is in flight when the block goes back
-  g_pinned.release(pin, nt * kPiece, tag);
+  g_copy_blocks.release(pin, pinned, tag);
   return e;
 }
 
@@ -579,7 +586,7 @@ struct Batch {
     const size_t extra = align256(sizeof(SpotDev) * n) + align256(sizeof(int2) * nb_all) + align256(sizeof(int) * n) +
                          align256(sizeof(int) * (size_t)n * kMaxInstances) + align256(sizeof(int2) * bnd_all);
     h_static_cap = align256(std::max<size_t>(static_bytes, 16)) + extra;
-    CU(g_pinned.acquire(h_static_cap, &h_static, &h_static_tag));
+    CU(g_pinned.acquire(&h_static_cap, &h_static, &h_static_tag));
     // ---- fill static ----
     h_spots.resize(n);
     std::vector<int2> work;
