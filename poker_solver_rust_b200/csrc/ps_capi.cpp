@@ -194,9 +194,9 @@ StreamPool g_streams;
 // a pinned block of their own each, so pieces are copied out while others
 // arrive.
 cudaError_t copy_out(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  constexpr size_t kPiece = 4u << 20;
+  constexpr size_t kPiece = 4u << 20, kThreads = 8;
   const size_t pieces = (bytes + kPiece - 1) / kPiece;
-  const size_t nt = std::min<size_t>({pieces, 8, std::max(1u, std::thread::hardware_concurrency())});
+  const size_t nt = std::min<size_t>({pieces, kThreads, std::max(1u, std::thread::hardware_concurrency())});
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -208,7 +208,7 @@ cudaError_t copy_out(void* dst, const void* src, size_t bytes, cudaStream_t s) {
     e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
     return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
   }
-  std::vector<cudaError_t> err(nt, cudaSuccess);
+  cudaError_t err[kThreads] = {};  // (nothing below throws while the block is held)
   auto work = [&](size_t t) {
     err[t] = cudaSetDevice(dev);
     for (size_t i = t; i < pieces && err[t] == cudaSuccess; i += nt) {
