@@ -233,6 +233,15 @@ cudaError_t copy_out(void* dst, const void* src, size_t bytes, cudaStream_t s) {
   return e;
 }
 
+// Pageable host to device memory, in the order of stream s; returns when it is
+// there.  (A plain cudaMemcpy of pageable memory may return before its last
+// part has arrived, and stream s, which does not wait for the default stream,
+// could then read the old values.)
+cudaError_t copy_in(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+  return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
 // Host arrays that copy_out fills: resizing one does not write its elements.
 template <class T>
 struct RawAllocator : std::allocator<T> {
@@ -2243,7 +2252,7 @@ int ps_seed_node_storage(ps_game* G, int64_t idx, int which, const float* v, int
     for (int h = 0; h < H; ++h) rows[(size_t)a * hs + h] = v[(size_t)a * H + h];
   const SpotDev& s = G->b->h_spots[0];
   float* dst = (which == 1 ? s.S : s.R) + nd.rs_off;
-  CU(cudaMemcpy(dst, rows.data(), 4 * rows.size(), cudaMemcpyHostToDevice));
+  CU(copy_in(dst, rows.data(), 4 * rows.size(), G->b->stream));
   G->host_dirty = true;
   return PS_OK;
 }
@@ -2324,7 +2333,7 @@ int ps_set_boundary_cfvs(ps_game* G, int64_t ordinal, int p, const float* cfvs, 
   if (G->state == GState::TreeBuilt) return fail(PS_ERR_STATE, "allocate memory before setting boundary values");
   G->bcfv_host[ordinal * 2 + p].assign(cfvs, cfvs + n);
   const SpotDev& s = G->b->h_spots[0];
-  CU(cudaMemcpy((float*)s.bcfv + ((size_t)ordinal * 2 + p) * g.vstride, cfvs, 4 * (size_t)n, cudaMemcpyHostToDevice));
+  CU(copy_in((float*)s.bcfv + ((size_t)ordinal * 2 + p) * g.vstride, cfvs, 4 * (size_t)n, G->b->stream));
   G->bcfv_set[ordinal * 2 + p] = 1;
   return PS_OK;
 }
@@ -2659,8 +2668,8 @@ int ps_state_import(ps_game* G, const void* buf, uint64_t size) {
   if (hdr[0] != 0x3153505342303032ull || hdr[1] != g.num_storage || size != 16 + 8 * g.num_storage)
     return fail(PS_ERR_INVALID, "storage size mismatch");
   const SpotDev& s = G->b->h_spots[0];
-  CU(cudaMemcpy(s.S, (const char*)buf + 16, 4 * g.num_storage, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(s.R, (const char*)buf + 16 + 4 * g.num_storage, 4 * g.num_storage, cudaMemcpyHostToDevice));
+  CU(copy_in(s.S, (const char*)buf + 16, 4 * g.num_storage, G->b->stream));
+  CU(copy_in(s.R, (const char*)buf + 16 + 4 * g.num_storage, 4 * g.num_storage, G->b->stream));
   G->host_dirty = true;
   return PS_OK;
 }
