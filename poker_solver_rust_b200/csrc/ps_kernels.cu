@@ -956,9 +956,9 @@ __device__ __noinline__ void run_pass_split(const Ctx& c, int p, const Discount 
       }
     }
     const int busy = cta_runs ? ng * nw0 : min(ng * TP, nb);
-    // node ops in up to 16 parts: a 1128-hand row is 282 float4 columns, so 9
-    // parts (cols) cover it in one round.  A step of more ops than warps takes
-    // the parts that waste least of its last round, and chance ops (48 children
+    // node ops in up to 16 parts: cols parts cover a row in one round (9 of a
+    // turn's 1128 hands, 10 of a flop's 1176).  A step of more ops than warps
+    // takes the parts that waste least of its last round, and chance ops (48 children
     // each) always go a round of columns to a warp: 60 iterations of the turn
     // game with its construction 93 -> 76 ms.
     const int cols = (sp.hs[p] + 127) >> 7;
@@ -968,7 +968,7 @@ __device__ __noinline__ void run_pass_split(const Ctx& c, int p, const Discount 
     if (ne > 0) P = 16 * ne <= nw - busy ? 16 : max(1, (nw - busy) / ne);
     if (P == 1 && ne > 1) {
       int best = ((ne + nw - 1) / nw) * cols;
-      for (int k = 2; k <= min(cols, 9); ++k) {
+      for (int k = 2; k <= min(cols, 16); ++k) {
         const int cost = ((ne * k + nw - 1) / nw) * ((cols + k - 1) / k);
         if (cost < best) {
           best = cost;
