@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -2357,17 +2358,22 @@ cudaError_t launch_grid(const SpotDev* spot, const GridJob& job, const Discount*
   if (grid < 2 || grid > 16) return cudaErrorInvalidValue;
   if ((e = grid_cluster_attrs()) != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = grid;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  // Shared memory for one CTA an SM, the rest of it as L1: sized for the most
+  // CTAs an SM could hold, as by default, the L1 depends on where the hand
+  // count falls between their steps (28 to 124 KB).
+  at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  at[1].val.sharedMemCarveout = (unsigned)std::min<size_t>(100, (smem + 2048) * 100 / (228 * 1024) + 1);
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelExC(&cfg, (const void*)k_grid, args);
 }
 
