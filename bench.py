@@ -318,7 +318,7 @@ def turn_datagen_measure(ps, spots, n: int, iters: int, interval: int):
     return {"workload": f"{n} depth-limited turn spots, {iters} iterations, boundary network re-evaluated every "
                         f"{interval} (7x500 bf16 MLP stand-in, 2720 -> 1326)",
             "boundary_items": bs.num_boundary_items(), "spots_per_s": n / best, "seconds": best,
-            "first_layer": "factored (ps_boundary_first_layer)",
+            "first_layer": "factored (ps_boundary_first_layer_cards)",
             "spots_per_s_dense_first_layer": n / dense,
             "mean_expl_pct_pot": float(np.mean(e / bs.starting_pots) * 100),
             "note": "host-timed end to end on the device: network (first layer factored over the river cards), "

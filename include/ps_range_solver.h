@@ -253,11 +253,13 @@ typedef struct ps_batch_opts {
                              -1 = autotune: time each shape on a sample of the batch) */
   int32_t ctas_per_sm;    /* 0 = as many as fit */
   int32_t sort_by_cost;   /* 1 = hand out the largest spots first */
-  int32_t stage_tables;   /* 1 = copy a spot's board tables to shared memory, 0 = read them
-                             from global memory, -1 = default (0) */
+  int32_t stage_tables;   /* 1 = copy a spot's board tables to shared memory (step-synchronous
+                             kernel), 0 = read them from global memory, -1 = default (0) */
   int32_t scan_buffers;   /* warps per CTA that evaluate terminal runs, each with a shared-memory
-                             scan buffer of 12 bytes per hand (0 = half the warps; the
-                             autotuner then also tries all of them) */
+                             scan buffer of about 12 bytes per hand (0 = half the warps; the
+                             autotuner then also tries all of them).  From 16 spots to one per
+                             SM, a number whose buffers do not fit in shared memory selects
+                             the step-synchronous kernel */
   int32_t instances_per_cta; /* spots of one tree shape a CTA solves in lockstep, 1..4
                                 (0 = 1); they share each step's barrier */
   int32_t scheduler;      /* PS_SCHED_DEFAULT (0): dataflow for batches of 16 spots or more

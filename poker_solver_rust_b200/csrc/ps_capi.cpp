@@ -454,8 +454,8 @@ struct Batch {
   int grid_cluster = 0;  // grid mode on the CTAs of one thread-block cluster (hardware barrier)
   unsigned* d_bar = nullptr;
   double* d_gred = nullptr;
-  // dataflow scheduler (k_flow) for solve and run_iterations; the adjoint
-  // and single spots keep the step-synchronous k_solve
+  // dataflow scheduler (k_flow) for solve, run_iterations and the adjoint;
+  // fewer than kFlowMinSpots spots keep the step-synchronous k_solve
   bool flow = false;
   int flow_block = 512, flow_grid = 0, flow_cps = 0, flow_lanes = 2, flow_parts = 1;
   SmemPlan flow_plan{};
@@ -756,8 +756,13 @@ struct Batch {
       if (sched < PS_SCHED_DEFAULT || sched > PS_SCHED_FLOW) return fail(PS_ERR_INVALID, "unknown scheduler");
       // the dataflow kernel is the faster one also where every spot has an SM
       // to itself (16 river spots 54 against 121 ms, 100: 69 against 155, 148:
-      // 66 against 153); a handful of spots, and a caller that shapes or tunes
-      // the step-synchronous CTAs of so few, keep that schedule
+      // 66 against 153; whole turn trees of 1128 hands, 10 iterations: 16 spots
+      // 60 against 207 ms, 148: 74 against 234; depth-limited turn spots, 30
+      // iterations: 16 spots 6.8 against 13.4 ms, 148: 8.5 against 18.9).  Spots
+      // of fewer than about 100 hands run within a tenth of each other (60
+      // iterations of 60 hands 3.15 against 2.93 to 3.10 ms).  A handful of
+      // spots, and a caller that shapes or tunes the step-synchronous CTAs of
+      // so few, keep that schedule
       const bool shaped = opts && (opts->block_threads != 0 || opts->ctas_per_sm > 0 || opts->instances_per_cta > 0 ||
                                    opts->stage_tables >= 0);
       flow = sched == PS_SCHED_FLOW ||

@@ -102,7 +102,7 @@ struct Ctx {
   float* buf;    // smem: this warp's scan buffer [scan_buf_floats(vstride)] (null for warps >= bufs)
   int bufs;      // warps 0 .. bufs-1 own a scan buffer
   int owner;     // >= 0: adjoint pass, terminal values are player owner's payoffs (see warp_terms)
-  int signed_reach;  // reach may be negative: terminal scans take segment starts from the bitmap
+  int signed_reach;  // the root reach is a caller's vector: the pass takes the general terminal copy (GEN)
   float* bgrad;  // boundary gradient buffer [num_boundary][2][vstride], or null
   float* breach; // boundary reach buffer [num_boundary][2][vstride] (reach of each player), or null
   double* red;   // smem: reduction scratch       [32]

@@ -89,7 +89,8 @@ cudaError_t launch_river_average_grad(int n, const ItemMeta& meta, const float* 
 // the sum of percard), percard [n][52][h] (weights times the reach of the
 // combos holding each card), wcols [68][h] (the board, rank, pot, stack and
 // player columns), bias [h] or null; out [n][2][48][h], f32 or bf16; h at most
-// kMaxFirstLayerWidth.
+// kMaxFirstLayerWidth, the documented range of the entry points (the kernel
+// takes columns in rounds and has no limit of its own).
 constexpr int kMaxFirstLayerWidth = 8192;
 cudaError_t launch_boundary_first_layer(int n, const ItemMeta& meta, const float* base, const float* percard,
                                         const float* wcols, const float* bias, int h, void* out, int bf16,
