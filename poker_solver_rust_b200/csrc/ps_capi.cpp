@@ -815,10 +815,12 @@ struct Batch {
           CU(dalloc(&d_gred, 64));
           // A small tree runs on one cluster of 16 CTAs instead, its steps
           // ended by the hardware cluster barrier: a river game of 33 nodes
-          // iterates 1.24x faster so, and datagen spots of 21-129 nodes solve
-          // 1.21-1.41x faster; from about 150k acting hand-edges per iteration
-          // the wider steps need the whole grid (a 141-node river tree with
-          // 1081 hands ran 3% slower on the cluster, a 357-node one 24%).
+          // iterates 1.30x faster so, and datagen spots of 21-129 nodes solve
+          // 1.21-1.41x faster; wider steps need the whole grid.  The line was
+          // drawn where the two forms of an earlier kernel met, at about 150k
+          // acting hand-edges per iteration; now a 129-node river tree with
+          // 1081 hands (138k) still runs 1.28x faster on the cluster and a
+          // 273-node one (294k) equally fast.
           // PS_GRID_CLUSTER = C overrides: 0 = never, 2..16 = always, on C CTAs.
           const Game& g0 = *games[0];
           int64_t S = 0;
