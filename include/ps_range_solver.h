@@ -254,7 +254,8 @@ typedef struct ps_batch_opts {
   int32_t ctas_per_sm;    /* 0 = as many as fit */
   int32_t sort_by_cost;   /* 1 = hand out the largest spots first */
   int32_t stage_tables;   /* 1 = copy a spot's board tables to shared memory (step-synchronous
-                             kernel), 0 = read them from global memory, -1 = default (0) */
+                             kernel, one spot per CTA), 0 = read them from global memory,
+                             -1 = default (0) */
   int32_t scan_buffers;   /* warps per CTA that evaluate terminal runs, each with a shared-memory
                              scan buffer of about 12 bytes per hand (0 = half the warps; the
                              autotuner then also tries all of them).  From 16 spots to one per

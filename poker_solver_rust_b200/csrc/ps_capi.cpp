@@ -744,7 +744,8 @@ struct Batch {
     plan.warps = block / 32;
     plan.bufs = opts && opts->scan_buffers > 0 ? std::min(opts->scan_buffers, plan.warps)
                                                : std::max(1, plan.warps / 2);
-    plan.tables = (single_board && stage == 1) ? table_bytes_for(hs_max, hs_max) : 0;
+    // (one spot's tables: spots in lockstep would overwrite each other's)
+    plan.tables = (single_board && stage == 1 && inst_k == 1) ? table_bytes_for(hs_max, hs_max) : 0;
     plan.split = n <= dc->nsm ? 1 : 0;  // a CTA per spot with an SM to itself: latency-bound
     int occ = solve_occupancy(block, plan);
     ctas_per_sm = opts && opts->ctas_per_sm > 0 ? std::min(opts->ctas_per_sm, occ) : occ;

@@ -146,3 +146,12 @@ def test_tuned_shape_that_does_not_fit_is_replaced():
         sp = _thin(200, seed=72, hands=hands)
         b = _batch(sp, block_threads=-1)
         _same(_solved(b, 10), _solved(_batch(sp, scheduler=STEP), 10))
+
+
+@pytest.mark.parametrize("n", [40, 320])
+def test_staged_tables_with_spots_in_lockstep(n):
+    """A CTA that solves several spots in lockstep has no room for each one's tables: results are those
+    of tables read from global memory."""
+    sp = _thin(n, seed=6, hands=120)
+    _same(_solved(_batch(sp, scheduler=STEP, instances_per_cta=4, stage_tables=1), 6),
+          _solved(_batch(sp, scheduler=STEP), 6))
